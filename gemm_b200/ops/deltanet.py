@@ -54,7 +54,7 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, cu_q: torch
         return conv_silu_ref(x, w, state, cu_q, seq_slots)
     out = torch.empty(t, ch, dtype=torch.bfloat16, device=x.device)
     rc = _native.cuda().gb_ssm_conv_silu(_p(x), _i(x.stride(0)), _p(w), _p(state), _p(cu_q), _p(seq_slots), _p(out), _i(ch), _i(ch),
-                                         _i(w.shape[1]), _i(cu_q.numel() - 1), _s())
+                                         _i(w.shape[1]), _i(cu_q.numel() - 1), _l(t), _s())
     _native.check(rc, "gb_ssm_conv_silu")
     return out
 

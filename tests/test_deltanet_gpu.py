@@ -30,6 +30,25 @@ def test_conv_silu_with_history():
     assert torch.equal(st_gpu[1].cpu(), st[1])            # a slot no sequence uses is untouched
 
 
+@pytest.mark.parametrize("ch,ck,wide,off", [(512, 4, 768, 0), (510, 4, 513, 0), (1036, 2, 1040, 4), (257, 8, 300, 3), (64, 3, 64, 0)])
+def test_conv_silu_tiles(ch, ck, wide, off):
+    """Tiles of 32 tokens: sequences at and around their edges (empty and shorter than the window among them), more than 32 sequences, rows that are not
+    8-byte aligned, other window lengths."""
+    torch.manual_seed(5)
+    lens = [31, 0, 32, 33, 1, 2, 64, 65, 0, 200] + [1] * 30 + [7, 40]
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    slots = torch.randperm(len(lens) + 2)[: len(lens)].to(torch.int32)
+    x = torch.randn(sum(lens), wide).bfloat16()
+    w, st = torch.randn(ch, ck), torch.randn(len(lens) + 2, ck - 1, ch)
+    st_gpu = st.clone().cuda()
+    ref = dn.conv_silu(x[:, off: off + ch], w, st, cu, slots)
+    got = dn.conv_silu(x.cuda()[:, off: off + ch], w.cuda(), st_gpu, cu.cuda(), slots.cuda())
+    # the same f32 sums in the same order: the results differ by the sigmoid's rounding, at most one step of bf16
+    assert (got.float().cpu() - ref.float()).abs().max() <= 2 ** -7 * ref.float().abs().max()
+    assert _rel(got, ref) < 2 ** -9
+    assert torch.equal(st_gpu.cpu(), st)
+
+
 @pytest.mark.parametrize("ds,ng,hv", [(64, 2, 4), (128, 2, 6)])
 def test_deltanet_recurrence(ds, ng, hv):
     torch.manual_seed(2)
