@@ -248,6 +248,16 @@ def test_router_logits_small_batch(t, e, k):
     assert got.dtype == torch.float32 and _rel(got, ref) < 1e-5
 
 
+@pytest.mark.parametrize("t,e,k", [(1, 1, 256), (9, 63, 8192), (16, 64, 4096), (8, 2, 2304), (148, 128, 4096)])
+def test_router_logits_narrow(t, e, k):
+    """Launches of less than a CTA per SM give a warp one row and two tokens (the last one is just past them): odd rows and tokens, rounds of K."""
+    torch.manual_seed(23)
+    h = torch.randn(t, k + 8, device="cuda").bfloat16()[:, :k]
+    w = (torch.randn(e, k, device="cuda") * 0.05).bfloat16()
+    got, ref = moe.router_logits(h, w), h.double() @ w.double().t()
+    assert _rel(got.double(), ref) < k ** 0.5 * 2 ** -23          # f32 sums of k products
+
+
 @pytest.mark.parametrize("t,local", [(1, None), (64, None), (256, None), (64, (32, 16)), (200, (0, 64))])
 def test_route_plan_single_kernel(t, local, monkeypatch):
     """Routing + plan in one launch equals the two separate ops."""
