@@ -12,10 +12,13 @@
 // Two kernels.  dn_chunk_prep_kernel (one CTA per chunk and value head, all chunks of all sequences in parallel) computes what
 // does not depend on the state: the normalised q / k, T (forward substitution, one thread per column), T V, -T diag(exp c) K, M,
 // diag(exp c) Q and the decayed keys, all as bf16 tiles in a workspace.  dn_chunk_scan_kernel (one CTA per sequence and value head)
-// walks the chunks in order with the state in registers as fp32 accumulator fragments: three products per chunk (U, O, the state
-// update), the gated RMSNorm of O, and the output.  The products are 64 x 128 x 128 at most and sit on a serial chain, so they
-// run on warp-level mma tiles with register accumulators (nvcuda::wmma, bf16 in, fp32 out) rather than on tcgen05: a TMEM round
-// trip per link of the chain would cost more than the tiles themselves.
+// walks the chunks in order: three products per chunk (U, O, the state update), the gated RMSNorm of O, and the output.  The products
+// are 64 x 128 x 128 at most and sit on a serial chain.  Written with the value index as the rows of every product (U^T, O^T, S), each
+// one's accumulator IS the next one's left operand, register for register, so a warp carries 16 values through all three without
+// meeting another warp or shared memory; only the right operands come from there (ldmatrix), the next chunk's copied while this one
+// is worked on.  Warp-level mma (bf16 in, fp32 out) rather than tcgen05: a TMEM round trip per link of the chain would cost more than
+// the tiles themselves.  3001 tokens, 32 heads: 929 us with every link staged through shared memory, 359 us in this form, bound by the
+// rate of the warp-level mma (1792 of them per chunk on one SM); the preparation 246 -> 184 us.
 //
 // The reference's counterpart is the chunked scan of cuda/llm/cuda_llm_runner.c:8128 (batch_deltanet_scan_f32) and its test
 // cuda/llm/scan/deltanet_chunk_test.c; the per-token recurrence is common/transformer.h:2829-2851.
@@ -34,7 +37,7 @@ constexpr int kDnD = 128;           // d_state
 constexpr int kDnLd = kDnD + 8;     // bf16 row stride of a 128-wide tile in shared memory (the pad spreads the rows over the banks)
 constexpr int kDnLc = kDnC + 8;     // bf16 row stride of a 64-wide tile
 constexpr int kDnLf = kDnD + 4;     // fp32 row stride of the 64 x 128 staging tile
-constexpr int kDnLo = kDnC;         // L (64 x 64, fp32) lives in the columns 64 .. 127 of the staging tile while T is solved
+constexpr int kDnLo = kDnC;         // L transposed (64 x 64, fp32) lives in the columns 64 .. 127 of the staging tile while T is solved
 constexpr int kDnThreads = 256;
 
 struct DnChunkArgs {
@@ -46,7 +49,7 @@ struct DnChunkArgs {
   // workspace: entry (chunk, head) at index chunk * dt_rank + head
   __nv_bfloat16* gq;     // [64][128]  exp(c_i) q_i
   __nv_bfloat16* nw;     // [64][128]  -(T diag(exp c) K)
-  __nv_bfloat16* uv;     // [64][128]  T V
+  __nv_bfloat16* uv;     // [128][64]  T V, transposed
   __nv_bfloat16* kdt;    // [128][64]  exp(c_last - c_j) k_j, transposed
   __nv_bfloat16* mqk;    // [64][64]   M
   float* glast;          // exp(c_last)
@@ -147,11 +150,6 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
   }
   __syncthreads();
   const float c_last = sc[kDnC - 1];
-  for (int idx = tid; idx < kDnC * kDnD; idx += kDnThreads) {
-    const int j = idx / kDnD, c = idx % kDnD;
-    sGKT[c * kDnLc + j] = __float2bfloat16(__expf(sc[j]) * __bfloat162float(sK[j * kDnLd + c]));
-  }
-
   // K K^T and Q K^T (64 x 64 x 128): warp w computes the tiles (m = w & 3, n = 2 (w >> 2) and the next)
   const int tm = warp & 3, tn0 = (warp >> 2) * 2;
   for (int pass = 0; pass < 2; ++pass) {
@@ -174,8 +172,8 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
     __syncthreads();
     for (int idx = tid; idx < kDnC * kDnC; idx += kDnThreads) {
       const int i = idx / kDnC, j = idx % kDnC;
-      if (pass == 0) {
-        sL[i * kDnLf + j] = (j < i) ? sb[i] * __expf(sc[i] - sc[j]) * sF[i * kDnLf + j] : 0.f;
+      if (pass == 0) {                  // row i of L^T: L_ji (K K^T is symmetric)
+        sL[i * kDnLf + j] = (i < j) ? sb[j] * __expf(sc[j] - sc[i]) * sF[i * kDnLf + j] : 0.f;
       } else {
         const float m = (j <= i) ? __expf(sc[i] - sc[j]) * sF[i * kDnLf + j] : 0.f;
         a.mqk[(ws * kDnC + i) * kDnC + j] = __float2bfloat16(m);
@@ -184,24 +182,78 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
     __syncthreads();
   }
 
-  // T = (I + L)^-1 diag(beta) by forward substitution, column by column: four adjacent lanes share a column (each a quarter of
-  // the inner sum; x_j = 0 above the diagonal, so the sum starts at the column's block of four)
-  {
-    const int col = tid >> 2, q = tid & 3, j0 = (col & ~3) + q;
+  // T = (I + L)^-1 diag(beta) by forward substitution: two warps, a thread per column, 16 rows at a time in registers (the rows above them come back
+  // from shared memory, a row of L^T serves 16 unknowns with four broadcast loads).  A thread's 2016 products are independent but for the 64 steps of
+  // the diagonal blocks; one column over four lanes with a shuffle pair per row had a chain of 64 x (16 products + 2 shuffles).  The other warps
+  // meanwhile form the operands that only need q, k and the decays.
+  if (warp < 2) {
+    const int col = tid;
     const float bcol = sb[col];
-    for (int i = 0; i < kDnC; ++i) {
-      float part = 0.f;
-      for (int j = j0; j < i; j += 4) part += sL[i * kDnLf + j] * sF[j * kDnLf + col];
-      part += __shfl_xor_sync(0xffffffffu, part, 1);
-      part += __shfl_xor_sync(0xffffffffu, part, 2);
-      if (q == 0) sF[i * kDnLf + col] = ((i == col) ? bcol : 0.f) - part;
-      __syncwarp();
+    for (int i0 = 0; i0 < kDnC; i0 += 16) {
+      float xr[16], part[16][4];                         // a row's products in four sums, by j & 3: short chains
+#pragma unroll
+      for (int i = 0; i < 16; ++i) part[i][0] = part[i][1] = part[i][2] = part[i][3] = 0.f;
+      for (int j0 = 0; j0 < i0; j0 += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float xj = sF[(j0 + u) * kDnLf + col];
+          const float4* l4 = reinterpret_cast<const float4*>(sL + (j0 + u) * kDnLf + i0);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const float4 l = l4[v];
+            part[4 * v][u] += l.x * xj; part[4 * v + 1][u] += l.y * xj; part[4 * v + 2][u] += l.z * xj; part[4 * v + 3][u] += l.w * xj;
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float xj = xr[j] = ((i0 + j == col) ? bcol : 0.f) - ((part[j][0] + part[j][1]) + (part[j][2] + part[j][3]));
+        const float4* l4 = reinterpret_cast<const float4*>(sL + (i0 + j) * kDnLf + i0);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          if (4 * v + 3 <= j) continue;
+          const float4 l = l4[v];
+          if (4 * v > j) part[4 * v][j & 3] += l.x * xj;
+          if (4 * v + 1 > j) part[4 * v + 1][j & 3] += l.y * xj;
+          if (4 * v + 2 > j) part[4 * v + 2][j & 3] += l.z * xj;
+          if (4 * v + 3 > j) part[4 * v + 3][j & 3] += l.w * xj;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        sF[(i0 + i) * kDnLf + col] = xr[i];
+        sT[(i0 + i) * kDnLc + col] = __float2bfloat16(xr[i]);
+      }
     }
-  }
-  __syncthreads();
-  for (int idx = tid; idx < kDnC * kDnC; idx += kDnThreads) {
-    const int i = idx / kDnC, j = idx % kDnC;
-    sT[i * kDnLc + j] = __float2bfloat16(sF[i * kDnLf + j]);
+  } else {
+    const int t2 = tid - 64;
+    for (int idx = t2; idx < kDnC * kDnD / 8; idx += kDnThreads - 64) {             // exp(c_i) q_i, 16 bytes at a time
+      const int i = idx / (kDnD / 8), c = 8 * (idx % (kDnD / 8));
+      const float e = __expf(sc[i]);
+      const uint4 r = *reinterpret_cast<const uint4*>(sQ + i * kDnLd + c);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&r);
+      uint4 o;
+      uint32_t* po = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { const float2 f = __bfloat1622float2(h2[u]); po[u] = pack_bf16x2(e * f.x, e * f.y); }
+      *reinterpret_cast<uint4*>(a.gq + ws * kDnC * kDnD + (size_t)i * kDnD + c) = o;
+    }
+    for (int idx = t2; idx < kDnD * kDnC / 8; idx += kDnThreads - 64) {             // keys transposed: eight tokens of one key column
+      const int c = idx % kDnD, j = 8 * (idx / kDnD);
+      float kv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) kv[u] = __bfloat162float(sK[(j + u) * kDnLd + c]);
+      uint4 og, od;
+      uint32_t* pg = reinterpret_cast<uint32_t*>(&og);
+      uint32_t* pd = reinterpret_cast<uint32_t*>(&od);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        pg[u] = pack_bf16x2(__expf(sc[j + 2 * u]) * kv[2 * u], __expf(sc[j + 2 * u + 1]) * kv[2 * u + 1]);
+        pd[u] = pack_bf16x2(__expf(c_last - sc[j + 2 * u]) * kv[2 * u], __expf(c_last - sc[j + 2 * u + 1]) * kv[2 * u + 1]);
+      }
+      *reinterpret_cast<uint4*>(sGKT + c * kDnLc + j) = og;
+      *reinterpret_cast<uint4*>(a.kdt + ws * kDnD * kDnC + (size_t)c * kDnC + j) = od;
+    }
   }
   __syncthreads();
 
@@ -224,40 +276,77 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
 #pragma unroll
     for (int m = 0; m < 4; ++m) wmma::store_matrix_sync(sF + (16 * m) * kDnLf + 16 * warp, acc[m], kDnLf, wmma::mem_row_major);
     __syncthreads();
-    __nv_bfloat16* dst = (pass == 0 ? a.uv : a.nw) + ws * kDnC * kDnD;
-    const float sign = pass == 0 ? 1.0f : -1.0f;
-    for (int idx = tid; idx < kDnC * kDnD; idx += kDnThreads) dst[idx] = __float2bfloat16(sign * sF[(idx / kDnD) * kDnLf + idx % kDnD]);
+    if (pass == 0) {                    // transposed: 16 values x 2 groups of eight tokens per warp step (whole 32-byte sectors)
+      __nv_bfloat16* dst = a.uv + ws * kDnC * kDnD;
+      for (int idx = tid; idx < kDnD * kDnC / 8; idx += kDnThreads) {
+        const int j = 8 * ((idx & 1) + 2 * (idx / (2 * kDnD))), v = (idx >> 1) % kDnD;
+        uint4 o;
+        uint32_t* po = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) po[u] = pack_bf16x2(sF[(j + 2 * u) * kDnLf + v], sF[(j + 2 * u + 1) * kDnLf + v]);
+        *reinterpret_cast<uint4*>(dst + (size_t)v * kDnC + j) = o;
+      }
+    } else {
+      __nv_bfloat16* dst = a.nw + ws * kDnC * kDnD;
+      for (int idx = tid; idx < kDnC * kDnD / 4; idx += kDnThreads) {
+        const float4 f = *reinterpret_cast<const float4*>(sF + (idx / (kDnD / 4)) * kDnLf + 4 * (idx % (kDnD / 4)));
+        *reinterpret_cast<uint2*>(dst + 4 * idx) = make_uint2(pack_bf16x2(-f.x, -f.y), pack_bf16x2(-f.z, -f.w));
+      }
+    }
     __syncthreads();
-  }
-
-  for (int idx = tid; idx < kDnC * kDnD; idx += kDnThreads) {
-    const int i = idx / kDnD, c = idx % kDnD;
-    a.gq[ws * kDnC * kDnD + idx] = __float2bfloat16(__expf(sc[i]) * __bfloat162float(sQ[i * kDnLd + c]));
-  }
-  for (int idx = tid; idx < kDnD * kDnC; idx += kDnThreads) {
-    const int c = idx / kDnC, j = idx % kDnC;
-    a.kdt[ws * kDnD * kDnC + idx] = __float2bfloat16(__expf(c_last - sc[j]) * __bfloat162float(sK[j * kDnLd + c]));
   }
   if (tid == 0) a.glast[ws] = __expf(c_last);
 }
 
-constexpr int kDnLt = kDnC + 4;     // fp32 row stride of U stored transposed (128 x 64) in the staging tile
-constexpr int kScanStage = (kDnC * kDnLf > kDnD * kDnLt ? kDnC * kDnLf : kDnD * kDnLt);
-constexpr int kScanSmem = (2 * kDnC * kDnLd + 2 * kDnD * kDnLc + kDnC * kDnLc + kDnD * kDnLd) * 2 + (kScanStage + 8 * 256) * 4;
+// One stage of the scan's operands in shared memory (bf16): exp(c) Q and -(T diag(exp c) K) [token][key], decayed keys [key][token], T V [value][token], M
+constexpr int kScanNw = kDnC * kDnLd, kScanKd = 2 * kDnC * kDnLd, kScanUv = kScanKd + kDnD * kDnLc, kScanM = kScanUv + kDnD * kDnLc;
+constexpr int kScanStage = kScanM + kDnC * kDnLc;
+constexpr int kScanSmem = 2 * kScanStage * 2 + kDnC * kDnLf * 4;
 
-__global__ void __launch_bounds__(kDnThreads)
+__device__ __forceinline__ void dn_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// The right operands of two neighbouring 8-column tiles for 16 k: rows n .. n + 15 of a tile stored [n][k]; `addr` is this lane's row address
+// (row (lane >> 4) * 8 + (lane & 7), k offset ((lane >> 3) & 1) * 8).
+__device__ __forceinline__ void dn_ldm(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void dn_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// accumulators of the column tiles 2j and 2j + 1 -> the left operand for k = 16 j .. 16 j + 15
+__device__ __forceinline__ void dn_to_a(uint32_t* a, const float* c0, const float* c1) {
+  a[0] = pack_bf16x2(c0[0], c0[1]); a[1] = pack_bf16x2(c0[2], c0[3]); a[2] = pack_bf16x2(c1[0], c1[1]); a[3] = pack_bf16x2(c1[2], c1[3]);
+}
+
+// c[0 .. 7] (16 x 64) += a (16 x 16 K) times 64 rows of a tile stored [n][k] with LD elements per row; the next k step's operands are requested before this
+// one's products.
+template <int K, int LD>
+__device__ __forceinline__ void dn_product(float (*c)[4], const uint32_t (*a)[4], uint32_t addr) {
+  uint32_t b[2][4][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) dn_ldm(b[0][p], addr + (uint32_t)(16 * p * LD) * 2);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k + 1 < K)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) dn_ldm(b[(k + 1) & 1][p], addr + (uint32_t)(16 * p * LD + 16 * (k + 1)) * 2);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      dn_mma(c[2 * p], a[k], b[k & 1][p][0], b[k & 1][p][1]);
+      dn_mma(c[2 * p + 1], a[k], b[k & 1][p][2], b[k & 1][p][3]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kDnThreads, 1)
 dn_chunk_scan_kernel(const DnChunkArgs a) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(128) uint8_t dn_smem[];
-  __nv_bfloat16* sGQ = reinterpret_cast<__nv_bfloat16*>(dn_smem);         // [64][kDnLd]
-  __nv_bfloat16* sNW = sGQ + kDnC * kDnLd;                                 // [64][kDnLd]
-  __nv_bfloat16* sKdT = sNW + kDnC * kDnLd;                                // [128][kDnLc]
-  __nv_bfloat16* sUT = sKdT + kDnD * kDnLc;                                // [128][kDnLc] U transposed
-  __nv_bfloat16* sMqk = sUT + kDnD * kDnLc;                                // [64][kDnLc]
-  __nv_bfloat16* sSb = sMqk + kDnC * kDnLc;                                // [128][kDnLd] the state as bf16, [value][key]
-  float* sF = reinterpret_cast<float*>(sSb + kDnD * kDnLd);                // [64][kDnLf]
-  float* sScr = sF + kScanStage;                                           // [8 warps][16 x 16]
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(dn_smem);        // [2][kScanStage]
+  float* sO = reinterpret_cast<float*>(ring + 2 * kScanStage);             // [64 tokens][kDnLf]
 
   const int h = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int seq_t0 = a.cu_q[s], seq_t1 = a.cu_q[s + 1];
@@ -266,120 +355,120 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
   for (int i = 0; i < s; ++i) cb += (a.cu_q[i + 1] - a.cu_q[i] + kDnC - 1) / kDnC;
   const int n_chunks = (seq_t1 - seq_t0 + kDnC - 1) / kDnC;
 
-  // state rows 16 warp .. of this head: eight 16 x 16 fp32 accumulator fragments per warp
-  float* st = a.state + ((size_t)a.seq_slots[s] * a.dt_rank + h) * kDnD * kDnD;
-  FragC S[8];
+  auto fetch = [&](int ci) {                                               // chunk ci -> its stage, 16 bytes per copy
+    const size_t ws = (size_t)(cb + ci) * a.dt_rank + h;
+    __nv_bfloat16* st = ring + (ci & 1) * kScanStage;
+    const __nv_bfloat16* gq = a.gq + ws * kDnC * kDnD;
+    const __nv_bfloat16* nw = a.nw + ws * kDnC * kDnD;
+    const __nv_bfloat16* kd = a.kdt + ws * kDnC * kDnD;
+    const __nv_bfloat16* uv = a.uv + ws * kDnC * kDnD;
+    const __nv_bfloat16* mq = a.mqk + ws * kDnC * kDnC;
 #pragma unroll
-  for (int f = 0; f < 8; ++f) wmma::load_matrix_sync(S[f], st + (16 * warp) * kDnD + 16 * f, kDnD, wmma::mem_row_major);
-  float* scr = sScr + warp * 256;
+    for (int i = 0; i < kDnC * kDnD / 8 / kDnThreads; ++i) {
+      const int idx = tid + i * kDnThreads;
+      const int r = idx / (kDnD / 8) * kDnLd + 8 * (idx % (kDnD / 8)), q = idx / (kDnC / 8) * kDnLc + 8 * (idx % (kDnC / 8));
+      dn_copy16(st + r, gq + 8 * idx);
+      dn_copy16(st + kScanNw + r, nw + 8 * idx);
+      dn_copy16(st + kScanKd + q, kd + 8 * idx);
+      dn_copy16(st + kScanUv + q, uv + 8 * idx);
+      if (i < kDnC * kDnC / 8 / kDnThreads) dn_copy16(st + kScanM + q, mq + 8 * idx);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
 
-  for (int ci = 0; ci < n_chunks; ++ci, ++cb) {
-    const size_t ws = (size_t)cb * a.dt_rank + h;
+  // state rows 16 warp .. of this head as accumulators: value rows g and g + 8, keys 8 f + 2 q and the next
+  const int g = lane >> 2, q = lane & 3;
+  float* st = a.state + ((size_t)a.seq_slots[s] * a.dt_rank + h) * kDnD * kDnD + (size_t)(16 * warp + g) * kDnD + 2 * q;
+  float S[16][4];
+#pragma unroll
+  for (int f = 0; f < 16; ++f) {
+    const float2 lo = *reinterpret_cast<const float2*>(st + 8 * f), hi = *reinterpret_cast<const float2*>(st + 8 * kDnD + 8 * f);
+    S[f][0] = lo.x; S[f][1] = lo.y; S[f][2] = hi.x; S[f][3] = hi.y;
+  }
+  const int lrow = (lane >> 4) * 8 + (lane & 7), lk = ((lane >> 3) & 1) * 8;
+  const uint32_t ring_u = smem_u32(ring);
+  const uint32_t off_d = (uint32_t)(lrow * kDnLd + lk) * 2, off_c = (uint32_t)(lrow * kDnLc + lk) * 2;
+  const float4 nwt = *reinterpret_cast<const float4*>(a.norm_w + 4 * lane);
+
+  for (int ci = 0; ci < n_chunks; ++ci) {
     const int t0 = seq_t0 + ci * kDnC, t1 = min(t0 + kDnC, seq_t1);
-    // the chunk's tiles -> shared memory (16 bytes per copy); T V goes to the staging tile as fp32: it is where U accumulates
-    {
-      const uint4* gq = reinterpret_cast<const uint4*>(a.gq + ws * kDnC * kDnD);
-      const uint4* nw = reinterpret_cast<const uint4*>(a.nw + ws * kDnC * kDnD);
-      const uint4* uv = reinterpret_cast<const uint4*>(a.uv + ws * kDnC * kDnD);
-      for (int idx = tid; idx < kDnC * kDnD / 8; idx += kDnThreads) {
-        const int i = idx / (kDnD / 8), v = idx % (kDnD / 8);
-        *reinterpret_cast<uint4*>(sGQ + i * kDnLd + 8 * v) = gq[idx];
-        *reinterpret_cast<uint4*>(sNW + i * kDnLd + 8 * v) = nw[idx];
-        const uint4 u = uv[idx];
-        const __nv_bfloat16* ub = reinterpret_cast<const __nv_bfloat16*>(&u);
-        float* d = sF + i * kDnLf + 8 * v;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) d[e] = __bfloat162float(ub[e]);
-      }
-      const uint4* kd = reinterpret_cast<const uint4*>(a.kdt + ws * kDnD * kDnC);
-      for (int idx = tid; idx < kDnD * kDnC / 8; idx += kDnThreads) {
-        const int c = idx / (kDnC / 8), v = idx % (kDnC / 8);
-        *reinterpret_cast<uint4*>(sKdT + c * kDnLc + 8 * v) = kd[idx];
-      }
-      const uint4* mq = reinterpret_cast<const uint4*>(a.mqk + ws * kDnC * kDnC);
-      for (int idx = tid; idx < kDnC * kDnC / 8; idx += kDnThreads) {
-        const int i = idx / (kDnC / 8), v = idx % (kDnC / 8);
-        *reinterpret_cast<uint4*>(sMqk + i * kDnLc + 8 * v) = mq[idx];
-      }
-    }
-    const float g_last = a.glast[ws];
-    // the state in front of the chunk as a bf16 operand
-#pragma unroll
-    for (int f = 0; f < 8; ++f) {
-      wmma::store_matrix_sync(scr, S[f], 16, wmma::mem_row_major);
-      __syncwarp();
-      for (int e = lane; e < 256; e += 32) sSb[(16 * warp + (e >> 4)) * kDnLd + 16 * f + (e & 15)] = __float2bfloat16(scr[e]);
-      __syncwarp();
-    }
-    __syncthreads();
+    const float g_last = a.glast[(size_t)(cb + ci) * a.dt_rank + h];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();          // this chunk's tiles have landed; everyone is done with the other stage and with sO
+    if (ci + 1 < n_chunks) fetch(ci + 1);
+    const __nv_bfloat16* stg = ring + (ci & 1) * kScanStage;
+    const uint32_t su = ring_u + (uint32_t)(ci & 1) * (kScanStage * 2);
 
-    // U = T V - (T diag(exp c) K) S0^T: warp w owns the value columns 16 w ..
-    {
-      FragC acc[4];
+    uint32_t aS[8][4];                                                     // the state in front of the chunk as a bf16 operand
 #pragma unroll
-      for (int m = 0; m < 4; ++m) wmma::load_matrix_sync(acc[m], sF + (16 * m) * kDnLf + 16 * warp, kDnLf, wmma::mem_row_major);
-      for (int kk = 0; kk < kDnD / 16; ++kk) {
-        FragB fb;
-        wmma::load_matrix_sync(fb, sSb + (16 * warp) * kDnLd + 16 * kk, kDnLd);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          FragA fa;
-          wmma::load_matrix_sync(fa, sNW + (16 * m) * kDnLd + 16 * kk, kDnLd);
-          wmma::mma_sync(acc[m], fa, fb, acc[m]);
-        }
-      }
-      __syncthreads();        // every warp has taken its columns of T V out of the staging tile: U goes back transposed, [value][token]
-#pragma unroll
-      for (int m = 0; m < 4; ++m) wmma::store_matrix_sync(sF + (16 * warp) * kDnLt + 16 * m, acc[m], kDnLt, wmma::mem_col_major);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < kDnD * kDnC; idx += kDnThreads) {
-      const int r = idx / kDnC, j = idx % kDnC;
-      sUT[r * kDnLc + j] = __float2bfloat16(sF[r * kDnLt + j]);
-    }
-    __syncthreads();
+    for (int k = 0; k < 8; ++k) dn_to_a(aS[k], S[2 * k], S[2 * k + 1]);
 
-    // O = diag(exp c) Q S0^T + M U
+    // U^T = (T V)^T - S0 (T diag(exp c) K)^T
+    uint32_t aU[4][4];
     {
-      FragC acc[4];
+      float U[8][4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) wmma::fill_fragment(acc[m], 0.f);
-      for (int kk = 0; kk < kDnD / 16; ++kk) {
-        FragB fb;
-        wmma::load_matrix_sync(fb, sSb + (16 * warp) * kDnLd + 16 * kk, kDnLd);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          FragA fa;
-          wmma::load_matrix_sync(fa, sGQ + (16 * m) * kDnLd + 16 * kk, kDnLd);
-          wmma::mma_sync(acc[m], fa, fb, acc[m]);
-        }
+      for (int n = 0; n < 8; ++n) {
+        const __nv_bfloat16* p = stg + kScanUv + (16 * warp + g) * kDnLc + 8 * n + 2 * q;
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + 8 * kDnLc));
+        U[n][0] = lo.x; U[n][1] = lo.y; U[n][2] = hi.x; U[n][3] = hi.y;
       }
-      for (int kk = 0; kk < kDnC / 16; ++kk) {
-        FragB fb;
-        wmma::load_matrix_sync(fb, sUT + (16 * warp) * kDnLc + 16 * kk, kDnLc);
+      dn_product<8, kDnLd>(U, aS, su + kScanNw * 2 + off_d);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          FragA fa;
-          wmma::load_matrix_sync(fa, sMqk + (16 * m) * kDnLc + 16 * kk, kDnLc);
-          wmma::mma_sync(acc[m], fa, fb, acc[m]);
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) wmma::store_matrix_sync(sF + (16 * m) * kDnLf + 16 * warp, acc[m], kDnLf, wmma::mem_row_major);
+      for (int k = 0; k < 4; ++k) dn_to_a(aU[k], U[2 * k], U[2 * k + 1]);
     }
-    __syncthreads();
+
+    // O^T = S0 (diag(exp c) Q)^T + U^T M^T
+    {
+      float O[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) O[n][e] = 0.f;
+      dn_product<8, kDnLd>(O, aS, su + off_d);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int p = k; p < 4; ++p) {                                      // M is lower triangular
+          uint32_t b[4];
+          dn_ldm(b, su + kScanM * 2 + off_c + (uint32_t)(16 * p * kDnLc + 16 * k) * 2);
+          dn_mma(O[2 * p], aU[k], b[0], b[1]);
+          dn_mma(O[2 * p + 1], aU[k], b[2], b[3]);
+        }
+      float* o = sO + 2 * q * kDnLf + 16 * warp + g;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        o[8 * n * kDnLf] = O[n][0]; o[(8 * n + 1) * kDnLf] = O[n][1];
+        o[8 * n * kDnLf + 8] = O[n][2]; o[(8 * n + 1) * kDnLf + 8] = O[n][3];
+      }
+    }
+    uint2 zr[8];                                                           // gates of the tokens this warp will finish
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + 8 * warp + i;
+      zr[i] = t < t1 ? *reinterpret_cast<const uint2*>(a.z + (size_t)t * a.ld_z + h * kDnD + 4 * lane) : make_uint2(0u, 0u);
+    }
+    __syncthreads();          // the output rows are complete
+
+    // S = exp(c_last) S + U^T diag(exp(c_last - c_j)) K
+#pragma unroll
+    for (int f = 0; f < 16; ++f)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[f][e] *= g_last;
+    dn_product<4, kDnLc>(S, aU, su + kScanKd * 2 + off_c);
+    dn_product<4, kDnLc>(S + 8, aU, su + (kScanKd + 64 * kDnLc) * 2 + off_c);
 
     // gated RMSNorm of the output rows: warp w takes the tokens 8 w .. 8 w + 7, a lane four features
-    for (int i = 8 * warp; i < 8 * warp + 8; ++i) {
-      const int t = t0 + i;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + 8 * warp + i;
       if (t >= t1) break;
-      const float4 o = *reinterpret_cast<const float4*>(sF + i * kDnLf + 4 * lane);
+      const float4 o = *reinterpret_cast<const float4*>(sO + (8 * warp + i) * kDnLf + 4 * lane);
       const float ss = dn_warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w);
       const float sc = rsqrtf(ss / (float)kDnD + a.eps);
-      const uint2 zr = *reinterpret_cast<const uint2*>(a.z + (size_t)t * a.ld_z + h * kDnD + 4 * lane);
-      const __nv_bfloat16* zb = reinterpret_cast<const __nv_bfloat16*>(&zr);
-      const float4 nw = *reinterpret_cast<const float4*>(a.norm_w + 4 * lane);
-      const float ov[4] = {o.x, o.y, o.z, o.w}, nv[4] = {nw.x, nw.y, nw.z, nw.w};
+      const __nv_bfloat16* zb = reinterpret_cast<const __nv_bfloat16*>(&zr[i]);
+      const float ov[4] = {o.x, o.y, o.z, o.w}, nv[4] = {nwt.x, nwt.y, nwt.z, nwt.w};
       __nv_bfloat16 y[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -388,26 +477,12 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
       }
       *reinterpret_cast<uint2*>(a.out + ((size_t)t * a.dt_rank + h) * kDnD + 4 * lane) = *reinterpret_cast<const uint2*>(y);
     }
-
-    // S = exp(c_last) S + U^T diag(exp(c_last - c_j)) K
-#pragma unroll
-    for (int f = 0; f < 8; ++f)
-#pragma unroll
-      for (int e = 0; e < S[f].num_elements; ++e) S[f].x[e] *= g_last;
-    for (int kk = 0; kk < kDnC / 16; ++kk) {
-      FragA fa;
-      wmma::load_matrix_sync(fa, sUT + (16 * warp) * kDnLc + 16 * kk, kDnLc);
-#pragma unroll
-      for (int f = 0; f < 8; ++f) {
-        FragB fb;
-        wmma::load_matrix_sync(fb, sKdT + (16 * f) * kDnLc + 16 * kk, kDnLc);
-        wmma::mma_sync(S[f], fa, fb, S[f]);
-      }
-    }
-    __syncthreads();          // the next chunk's tiles overwrite what this one still read
   }
 #pragma unroll
-  for (int f = 0; f < 8; ++f) wmma::store_matrix_sync(st + (16 * warp) * kDnD + 16 * f, S[f], kDnD, wmma::mem_row_major);
+  for (int f = 0; f < 16; ++f) {
+    *reinterpret_cast<float2*>(st + 8 * f) = make_float2(S[f][0], S[f][1]);
+    *reinterpret_cast<float2*>(st + 8 * kDnD + 8 * f) = make_float2(S[f][2], S[f][3]);
+  }
 }
 
 // bytes of one workspace entry (chunk, head): three 64 x 128 tiles, one 128 x 64, one 64 x 64 (bf16) and the chunk's total decay
