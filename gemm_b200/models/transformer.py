@@ -25,6 +25,7 @@ import os
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import _native
@@ -212,45 +213,58 @@ class ForwardBatch:
               stage: bool = False) -> "ForwardBatch":
         """Host-side assembly from per-sequence chunk lengths and the lengths already cached.  ``stage`` (INT8 KV cache) also lays the
         step's tokens out in the staging buffer: a decode step row by row, a prefill step with every sequence on a page boundary."""
+        # Whole arrays instead of a Python step per token (16384 tokens in 8 prompts: 34 ms), and one copy to the device for all of them.
         b = len(q_lens)
-        pos, slots, cu = [], [], [0]
-        bt = block_table.cpu()
-        for s in range(b):
-            for i in range(q_lens[s]):
-                p = ctx_lens[s] + i
-                pos.append(p)
-                slots.append(int(bt[s, p // page_size]) * page_size + p % page_size)
-            cu.append(cu[-1] + q_lens[s])
-        t = cu[-1]
-        rows = list(range(t)) if all_logits else [cu[s + 1] - 1 for s in range(b) if q_lens[s] > 0]
+        ql, ctx = np.asarray(q_lens, dtype=np.int64).reshape(b), np.asarray(ctx_lens, dtype=np.int64)[:b].reshape(b)
+        cu = np.concatenate([np.zeros(1, np.int64), np.cumsum(ql)])
+        t = int(cu[-1])
+        seq = np.repeat(np.arange(b), ql)
+        inside = np.arange(t) - cu[:-1][seq]                       # index of a token in its sequence's chunk
+        pos = ctx[seq] + inside
+        slots = block_table.cpu().numpy()[seq, pos // page_size].astype(np.int64) * page_size + pos % page_size
+        rows = np.arange(t) if all_logits else cu[1:][ql > 0] - 1
         i32 = dict(dtype=torch.int32, device=device)
         ids_t = ids.to(device=device, dtype=torch.int32) if torch.is_tensor(ids) else torch.tensor(ids, **i32)
-        st_slots = st_bt = None
+        parts = dict(positions=pos, slots=slots, cu_q=cu, kv_len=ctx + ql, work=att.build_work(q_lens, hq, hkv, num_splits).numpy(),
+                     seq_slots=np.asarray([int(x) for x in seq_slots] if seq_slots is not None else range(b), dtype=np.int64))
+        if block_table.device.type == "cpu" and torch.device(device).type != "cpu":
+            parts["block_table"] = block_table.numpy()
         if stage:
             if all(q == 1 for q in q_lens):
-                st_slots = torch.arange(t, **i32)
+                parts["stage_slots"] = np.arange(t)
             else:
                 if any(c != 0 for c in ctx_lens):
                     raise NotImplementedError("INT8 KV cache: a prefill chunk must start its sequence (the attention of a later chunk "
                                               "would have to read the quantised history; raise max_prefill_tokens or use the bf16 cache)")
-                pages = [(q + page_size - 1) // page_size for q in q_lens]
-                first, ss = [0], []
-                for s in range(b):
-                    ss.extend(first[s] * page_size + i for i in range(q_lens[s]))
-                    first.append(first[s] + pages[s])
-                st_slots = torch.tensor(ss, **i32)
-                st_bt = torch.zeros(b, max(max(pages), 1), dtype=torch.int32)
-                for s in range(b):
-                    st_bt[s, : pages[s]] = torch.arange(first[s], first[s] + pages[s], dtype=torch.int32)
-                st_bt = st_bt.to(device)
-        return ForwardBatch(stage_slots=st_slots, stage_bt=st_bt, plans={}, q_lens=list(q_lens), kv_lens=[c + q for c, q in zip(ctx_lens, q_lens)],
-                            ids=ids_t, positions=torch.tensor(pos, **i32), slots=torch.tensor(slots, **i32),
-                            cu_q=torch.tensor(cu, **i32), kv_len=torch.tensor([c + q for c, q in zip(ctx_lens, q_lens)], **i32),
-                            block_table=block_table.to(device=device, dtype=torch.int32),
-                            work=att.build_work(q_lens, hq, hkv, num_splits).to(device),
-                            logit_rows=torch.tensor(rows, dtype=torch.int64, device=device), num_splits=num_splits, n_tokens=t,
-                            seq_slots=torch.tensor(list(seq_slots) if seq_slots is not None else list(range(b)), **i32),
-                            is_decode=(b > 0 and all(q == 1 for q in q_lens)))
+                pages = (ql + page_size - 1) // page_size
+                first = np.cumsum(pages) - pages
+                parts["stage_slots"] = first[seq] * page_size + inside
+                col = np.arange(max(int(pages.max(initial=0)), 1))
+                parts["stage_bt"] = np.where(col < pages[:, None], first[:, None] + col, 0)
+        dev = _to_device(rows, parts, device)
+        if "block_table" not in dev:
+            dev["block_table"] = block_table.to(device=device, dtype=torch.int32)
+        return ForwardBatch(plans={}, q_lens=list(q_lens), kv_lens=[c + q for c, q in zip(ctx_lens, q_lens)], ids=ids_t, num_splits=num_splits, n_tokens=t,
+                            is_decode=(b > 0 and all(q == 1 for q in q_lens)), **dev)
+
+
+def _to_device(rows: np.ndarray, parts: dict, device) -> dict:
+    """The arrays as int32 tensors (and ``rows`` as int64 ``logit_rows``): 16-byte aligned views of one buffer that is copied once."""
+    at = -(-2 * rows.size // 4) * 4                               # `rows` in front, in pairs of 32-bit words
+    where = {}
+    for name, a in parts.items():
+        where[name] = at
+        at += -(-a.size // 4) * 4
+    host = np.zeros(at, np.int32)
+    host[: 2 * rows.size] = np.ascontiguousarray(rows, dtype=np.int64).view(np.int32)
+    for name, a in parts.items():
+        if a.size and (a.max() > 2 ** 31 - 1 or a.min() < -2 ** 31):
+            raise RuntimeError(f"{name}: value cannot be converted to int32 without overflow")
+        host[where[name]: where[name] + a.size] = a.reshape(-1)
+    buf = torch.from_numpy(host).to(device)
+    out = {name: buf[where[name]: where[name] + a.size].view(a.shape) for name, a in parts.items()}
+    out["logit_rows"] = buf[: 2 * rows.size].view(torch.int64)
+    return out
 
 
 def attention_plan(q_lens: Sequence[int], max_kv: int, hq: int, hkv: int, span: int, device, decode: bool):

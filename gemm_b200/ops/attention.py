@@ -11,8 +11,9 @@ from __future__ import annotations
 import ctypes
 import math
 import os
-from typing import List, Optional, Sequence
+from typing import Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import _native
@@ -34,14 +35,11 @@ def build_work(q_lens: Sequence[int], hq: int, hkv: int, num_splits: int = 1) ->
     tpt = 128 // g
     if tpt == 0:                          # more query heads per KV head than a tile has rows: no work for the tcgen05 kernels
         return torch.zeros(0, 4, dtype=torch.int32)
-    items: List[List[int]] = []
-    for s, ql in enumerate(q_lens):
-        n_tiles = (ql + tpt - 1) // tpt
-        for ti in reversed(range(n_tiles)):
-            for sp in range(num_splits):
-                for h in range(hkv):
-                    items.append([s, h, ti * tpt, sp])
-    return torch.tensor(items, dtype=torch.int32).reshape(-1, 4)
+    tiles = np.maximum((np.asarray(q_lens, dtype=np.int64) + (tpt - 1)) // tpt, 0)
+    seq = np.repeat(np.arange(len(tiles)), tiles * (num_splits * hkv))
+    at = np.arange(len(seq)) - np.repeat(np.cumsum(tiles) - tiles, tiles * (num_splits * hkv)) * (num_splits * hkv)       # item of its sequence: (tile, split, head)
+    tile = tiles[seq] - 1 - at // (num_splits * hkv)
+    return torch.from_numpy(np.stack([seq, at % hkv, tile * tpt, at // hkv % num_splits], 1).astype(np.int32))
 
 
 def pick_splits(n_seqs: int, hkv: int, max_kv: int, sm_count: int = 148, ctas_per_sm: int = 2) -> int:

@@ -179,7 +179,7 @@ class Engine:
                 q_lens.append(take); ctx.append(done[i]); seqs.append(i)
                 ids.append(prompts[i][done[i]:done[i] + take])
                 room -= take
-            fb = ForwardBatch.build(q_lens, ctx, torch.cat([x.to(self.device) for x in ids]), self._block_table([base + i for i in seqs]),
+            fb = ForwardBatch.build(q_lens, ctx, torch.cat(ids if all(x.device.type == "cpu" for x in ids) else [x.to(self.device) for x in ids]), self._block_table([base + i for i in seqs]),
                                     self.page_size, self.hq_local, self.hkv_local, self.device, seq_slots=[base + i for i in seqs],
                                     stage=self.kv.quantized)
             if embeds is not None:
