@@ -24,6 +24,7 @@
 #include "host_common.h"
 #include <stdlib.h>
 #include "../fabric/fabric.cuh"
+#include "gemm_pair.cuh"
 
 namespace gb {
 
@@ -905,6 +906,19 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
   a.tile_hint = num_groups == 0 ? max_tiles : num_groups * ((n_out + 127) / 128);
   a.m_tok_hint = num_groups == 0 ? m_tok : (tn <= 32 ? tn : 1 << 20);
   if (num_groups == 0 && m_tok <= 0) return 0;
+
+  // SiLU gate / up projections of more than 64 tokens run on SM pairs (gemm_pair.cuh says why, and what both sides measure)
+  if (dual && !mx && !qo && tn >= 128 && num_groups == 0 && n_out % 256 == 0 && up_row_offset % 128 == 0 && a.splits <= 1 && row_map == nullptr &&
+      row_scale == nullptr && bias == nullptr && a.amax_val == nullptr && !a.out_f32 && !gelu && !capped && !a.dual_raw && a.wait_n == 0 &&
+      a.peer_region_rows == 0 && a.peer_bcast == 0 && a.signal_n == 0 && a.out_bytes != 0) {
+    CUtensorMap tmH;
+    if (make_tmap_2d(&tmH, x, dt, (uint64_t)k, (uint64_t)x_rows, (uint64_t)ldx * esz, box_k, 128, TM_SW_128)) return -1;
+    PairArgs pa;
+    memset(&pa, 0, sizeof(pa));
+    pa.m_tok = m_tok; pa.num_kb = (k + 63) / 64; pa.up_row_offset = up_row_offset; pa.out = (__nv_bfloat16*)out; pa.ldo = ldo;
+    pa.out_bytes = a.out_bytes; pa.w_tiled = a.w_tiled; pa.status = a.status;
+    return launch_gemm_pair(tmW, tmH, n_out, pa, stream);
+  }
 
   if (a.silu_rows > 0) {
     if (tn == 128) return launch_gemm<128, 0, false, false, 1>(tmW, tmX, a, max_tiles, stream);

@@ -1,0 +1,38 @@
+"""Prefill-sized bf16 gate / up projections (tiles of 256 features x up to 256 tokens on SM pairs) against f32 products, at the edges of tiles, of the K steps
+and of the rings, for one to many tiles per pair."""
+import pytest
+import torch
+
+from gemm_b200 import _native
+from gemm_b200.ops import gemm, mxfp8
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(65, 256, 64), (96, 256, 4096), (129, 512, 128), (257, 512, 72), (300, 768, 320), (511, 256, 1024), (2049, 1024, 520), (288, 4096, 4096), (5000, 1280, 256),
+          (2600, 6144, 448)]
+
+
+def _inputs(m, n, k):
+    torch.manual_seed(m + n + k)
+    x = torch.randn(m, k + 8, device="cuda").bfloat16()[:, :k]               # rows wider than the operand
+    w = (torch.randn(n, k, device="cuda") * k ** -0.5).bfloat16()
+    return x, w
+
+
+def _close(got, ref):
+    # f32 sums of exact bf16 products, then one rounding to bf16 (f32 results: none)
+    _native.assert_status_ok()
+    bound = ref.abs() * (2 ** -8 if got.dtype == torch.bfloat16 else 0) + 1e-4
+    assert ((got.float() - ref).abs() <= bound).all(), (got.float() - ref).abs().max()
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_swiglu(m, n, k):
+    x, w = _inputs(m, 2 * n, k)
+    y = x.float() @ w.float().t()
+    ref = torch.nn.functional.silu(y[:, :n]) * y[:, n:]
+    tiled = k % 64 == 0
+    out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.linear_swiglu(x, mxfp8.tile_weight(w) if tiled else w, out=out[:m], w_tiled=tiled)
+    _close(out[:m], ref)
+    assert (out[m] == 7).all()
