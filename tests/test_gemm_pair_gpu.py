@@ -1,5 +1,5 @@
-"""Prefill-sized bf16 gate / up projections (tiles of 256 features x up to 256 tokens on SM pairs) against f32 products, at the edges of tiles, of the K steps
-and of the rings, for one to many tiles per pair."""
+"""Prefill-sized bf16 layers against f32 products, at the edges of tiles, of the K steps and of the rings: gate / up projections on SM pairs (256 features x up
+to 256 tokens, one to many tiles per pair), plain ones with more blocks of features than SMs (groups of eight token tiles)."""
 import pytest
 import torch
 
@@ -10,6 +10,7 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [(65, 256, 64), (96, 256, 4096), (129, 512, 128), (257, 512, 72), (300, 768, 320), (511, 256, 1024), (2049, 1024, 520), (288, 4096, 4096), (5000, 1280, 256),
           (2600, 6144, 448)]
+WIDE = [(256, 18944, 64), (300, 18951, 128), (2048, 19200, 192), (2305, 24576, 64), (4500, 18944, 72)]
 
 
 def _inputs(m, n, k):
@@ -34,5 +35,20 @@ def test_swiglu(m, n, k):
     tiled = k % 64 == 0
     out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
     gemm.linear_swiglu(x, mxfp8.tile_weight(w) if tiled else w, out=out[:m], w_tiled=tiled)
+    _close(out[:m], ref)
+    assert (out[m] == 7).all()
+
+
+@pytest.mark.parametrize("m,n,k", WIDE)
+@pytest.mark.parametrize("tiled", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_linear_with_many_features(m, n, k, tiled, dtype):
+    x, w = _inputs(m, n, k)
+    bias = torch.randn(n, device="cuda") if m % 2 else None
+    ref = x.float() @ w.float().t() + (bias if bias is not None else 0)
+    if tiled and (k % 64 or n % 128):
+        pytest.skip("tiled weights have whole blocks")
+    out = torch.full((m + 1, n), 7.0, dtype=dtype, device="cuda")
+    gemm.linear(x, mxfp8.tile_weight(w) if tiled else w, bias=bias, out=out[:m], w_tiled=tiled)
     _close(out[:m], ref)
     assert (out[m] == 7).all()
