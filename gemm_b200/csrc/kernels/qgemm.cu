@@ -284,18 +284,325 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const QGemmArgs args) {
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
 }
 
+// ------------------------------------------------------------------------------------------------------------------------------------------
+// More than 64 tokens.  The kernel above is then bound by shared memory: per 128 x 128 step of W it writes 32 KB of unpacked operand, and the MMAs read that and
+// the tokens' 32 KB again, 1470 cycles of the SM's shared memory for 512 of the tensor core, and every 128 tokens unpack W anew.  Here the unpacked operand never
+// meets shared memory: eight warps (a thread per weight row and 64-value chunk) write it straight into TMEM (tcgen05.st) and the MMA takes its A operand from
+// there; the token tile is up to 256 wide, so W is unpacked once per 256 tokens.  Same operands, same order of sums as above.  Qwen3-32B's four projections of
+// 512 tokens: QW_MEASURED.
+//
+// TMEM: columns 0-255 accumulators (one of up to 256 columns, or two of up to 128), 256-511 four operand stages of 128 rows x 128 bf16 (64 columns each).
+// Roles (576 threads): warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue (token half (warp - 2) / 4), warps 10-17 unpack (chunk (warp - 10) / 4 of a stage).
+constexpr int kQwThreads = 576;
+constexpr int kQwA = 4;                    // operand stages in TMEM
+// Stages of 64 token columns (32 KB each) and raw tiles (18 KB Q4_K, 34 KB Q8_0) in flight: what shared memory holds, the tokens' bytes first.
+__host__ __device__ constexpr int qw_b_stages(int type) { return type == 0 ? 5 : 4; }
+__host__ __device__ constexpr int qw_raw_stages(int type) { return type == 0 ? 3 : 2; }
+
+struct QWideArgs {
+  QGemmArgs g;
+  int tn;                                  // tokens of a tile: a multiple of 16, at most 256
+};
+
+template <int TYPE>
+__global__ void __launch_bounds__(kQwThreads, 1)
+qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs) {
+  constexpr int RAW = TYPE == 0 ? 128 * 144 : 128 * 272;
+  constexpr int RAW_PAD = (RAW + 1023) & ~1023;
+  constexpr int RS = qw_raw_stages(TYPE), BS = qw_b_stages(TYPE);
+  const QGemmArgs& args = wargs.g;
+  const int TN = wargs.tn, b_bytes = TN * 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* Bb = smem;                                    // [BS][256 rows][128 B]
+  uint8_t* rawb = smem + BS * 32768;                     // [RS][RAW_PAD]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(rawb + RS * RAW_PAD);
+  uint64_t* raw_full = bars;            // [RS]
+  uint64_t* raw_empty = raw_full + RS;  // [RS]  8 arrivals (unpack warps)
+  uint64_t* a_full = raw_empty + RS;    // [kQwA]  8 arrivals
+  uint64_t* a_empty = a_full + kQwA;    // [kQwA]  1 (commit)
+  uint64_t* b_full = a_empty + kQwA;    // [BS]
+  uint64_t* b_empty = b_full + BS;      // [BS]  1 (commit)
+  uint64_t* accf = b_empty + BS;        // [2]
+  uint64_t* acce = accf + 2;            // [2]  8 arrivals (epilogue warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acce + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_tiles = args.row_tiles * args.tok_tiles * args.splits;
+  const int nacc = TN <= 128 ? 2 : 1;
+  // token tiles vary fastest: the CTAs that run together share a tile of W
+  auto tile_at = [&](int t, int& rt, int& tb, int& kb0, int& kb1) {
+    const int ksp = t % args.splits, tt = t / args.splits;
+    tb = tt % args.tok_tiles; rt = tt / args.tok_tiles;
+    kb0 = ksp * args.kb_per; kb1 = min(args.num_kb, kb0 + args.kb_per);
+    return ksp;
+  };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
+    for (int i = 0; i < kQwA; ++i) { mbar_init(&a_full[i], 8); mbar_init(&a_empty[i], 1); }
+    for (int i = 0; i < BS; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&accf[i], 1); mbar_init(&acce[i], 8); }
+    *abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + 256;
+  pdl_wait();
+  pdl_trigger();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (lane == 0) {
+      int rs = 0; uint32_t rph = 0; int bs = 0; uint32_t bph = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
+        int rt, tb, kb0, kb1;
+        tile_at(t, rt, tb, kb0, kb1);
+        const uint8_t* wt = args.w + (size_t)rt * args.num_kb * RAW;
+        for (int kb = kb0; ok && kb < kb1; ++kb) {
+          if (!mbar_wait(&raw_empty[rs], rph ^ 1, abort_flag, args.status, 1240, rs)) { ok = false; break; }
+          mbar_expect_tx(&raw_full[rs], RAW);
+          bulk_load(rawb + rs * RAW_PAD, wt + (size_t)kb * RAW, RAW, &raw_full[rs]);
+          if (++rs == RS) { rs = 0; rph ^= 1; }
+          for (int h = 0; h < 4; ++h) {
+            if (!mbar_wait(&b_empty[bs], bph ^ 1, abort_flag, args.status, 1241, bs)) { ok = false; break; }
+            mbar_expect_tx(&b_full[bs], b_bytes);
+            tma_load_2d(Bb + bs * 32768, &tmX, &b_full[bs], kb * 256 + h * 64, tb * TN);
+            if (++bs == BS) { bs = 0; bph ^= 1; }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      int as = 0; uint32_t aph = 0; int bs = 0; uint32_t bph = 0; int acc = 0; uint32_t acc_ph = 0;
+      bool ok = true;
+      const uint32_t idesc = make_idesc(128, TN, 1, 1);
+      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
+        int rt, tb, kb0, kb1;
+        tile_at(t, rt, tb, kb0, kb1);
+        if (!mbar_wait(&acce[acc], acc_ph ^ 1, abort_flag, args.status, 1250, acc)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d0 = tmem_base + acc * 128;
+        for (int ks = 0; ok && ks < 2 * (kb1 - kb0); ++ks) {
+          if (!mbar_wait(&a_full[as], aph, abort_flag, args.status, 1251, as)) { ok = false; break; }
+          for (int half = 0; half < 2; ++half) {
+            if (!mbar_wait(&b_full[bs], bph, abort_flag, args.status, 1252, bs)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t b = make_sdesc_sw128(smem_u32(Bb + bs * 32768));
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              mma_f16_ts(d0, tmem_a + as * 64 + half * 32 + j * 8, sdesc_at(b, j * 32), idesc, (ks > 0 || half > 0 || j > 0) ? 1u : 0u);
+            tc_commit(&b_empty[bs]);
+            if (++bs == BS) { bs = 0; bph ^= 1; }
+          }
+          if (!ok) break;
+          tc_commit(&a_empty[as]);
+          if (++as == kQwA) { as = 0; aph ^= 1; }
+        }
+        if (!ok) break;
+        tc_commit(&accf[acc]);
+        if (++acc == nacc) { acc = 0; acc_ph ^= 1; }
+      }
+    }
+  } else if (warp < 10) {
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    const int q = warp & 3, c0 = ((warp - 2) >> 2) * 128;
+    int acc = 0; uint32_t acc_ph = 0;
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+      int rt, tb, kb0, kb1;
+      const int ksp = tile_at(t, rt, tb, kb0, kb1);
+      if (!__all_sync(0xffffffffu, mbar_wait(&accf[acc], acc_ph, abort_flag, args.status, 1260, acc))) break;
+      tc_fence_after();
+      const uint32_t tacc = tmem_base + acc * 128 + c0 + ((uint32_t)(q * 32) << 16);
+      const int n = rt * 128 + q * 32 + lane;
+      const bool n_ok = n < args.n_out;
+      const float bias = (args.bias != nullptr && n_ok && ksp == 0) ? args.bias[n] : 0.f;
+      const int tok0 = tb * TN + c0, live = min(min(128, TN - c0), args.m_tok - tok0);        // this warp's tokens (may be <= 0)
+      const size_t off0 = (size_t)ksp * (size_t)args.partial_stride + (size_t)tok0 * args.ldo + n;
+      if (!args.out_f32) {
+        // everything out of TMEM as packed bf16 before the stores: a 256-token tile has no second accumulator to go on with
+        uint32_t pk[64];
+#pragma unroll
+        for (int c = 0; c < 128; c += 16) {
+          if (c < live) {
+            uint32_t r[16];
+            tmem_ld_x16(tacc + c, r);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) pk[c / 2 + j] = pack_bf16x2(__uint_as_float(r[2 * j]) + bias, __uint_as_float(r[2 * j + 1]) + bias);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acce[acc]);
+        if (n_ok) {
+          unsigned short* o = reinterpret_cast<unsigned short*>(args.out) + off0;
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            if (2 * i < live) o[(size_t)(2 * i) * args.ldo] = (unsigned short)(pk[i] & 0xffffu);
+            if (2 * i + 1 < live) o[(size_t)(2 * i + 1) * args.ldo] = (unsigned short)(pk[i] >> 16);
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < live; c += 16) {
+          uint32_t r[16];
+          tmem_ld_x16(tacc + c, r);
+          tc_wait_ld();
+          if (!n_ok) continue;
+          float* o = reinterpret_cast<float*>(args.out) + off0 + (size_t)c * args.ldo;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) if (c + j < live) o[(size_t)j * args.ldo] = __uint_as_float(r[j]) + bias;
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acce[acc]);
+      }
+      if (++acc == nacc) { acc = 0; acc_ph ^= 1; }
+    }
+  } else {
+    // ------------------------------------------------------------------ unpack (warps 10..17): raw blocks -> operand in TMEM
+    const int q = warp & 3, part = (warp - 10) >> 2, row = q * 32 + lane;
+    const uint32_t ta = tmem_a + part * 32 + ((uint32_t)(q * 32) << 16);
+    int rs = 0; uint32_t rph = 0; int as = 0; uint32_t aph = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
+      int rt, tb, kb0, kb1;
+      tile_at(t, rt, tb, kb0, kb1);
+      for (int kb = kb0; ok && kb < kb1; ++kb) {
+        // warp-uniform, as are all steps below (stores to TMEM are a warp's)
+        if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rs], rph, abort_flag, args.status, 1270, rs))) { ok = false; break; }
+        const uint8_t* rb = rawb + rs * RAW_PAD;
+        uint32_t oo[2][32];                                // both stages of the tile, two values a word, in k order
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int j = 2 * h + part;                      // 64-value chunk of the 256-column tile
+          uint32_t* o = oo[h];
+          if (TYPE == 0) {
+            const uint8_t* b = rb + row * 144;
+            const uint4 hd = *reinterpret_cast<const uint4*>(b);
+            const uint4 q0 = *reinterpret_cast<const uint4*>(b + 16 + 32 * j), q1 = *reinterpret_cast<const uint4*>(b + 32 + 32 * j);
+            const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
+            const float d = __low2float(dd), dmin = __high2float(dd);
+            const int bsh = 16 * part;
+            uint32_t sc, mn;                               // two bytes: sub-blocks 2 j (low nibbles) and 2 j + 1 (high)
+            if (h == 0) { sc = (hd.y >> bsh) & 0x3f3fu; mn = (hd.z >> bsh) & 0x3f3fu; }
+            else {
+              const uint32_t x = hd.w >> bsh, y = hd.y >> bsh, z = hd.z >> bsh;
+              sc = (x & 0x0f0fu) | ((y >> 2) & 0x3030u); mn = ((x >> 4) & 0x0f0fu) | ((z >> 2) & 0x3030u);
+            }
+            const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+            const __nv_bfloat162 sixteen = __float2bfloat162_rn(16.0f);
+#pragma unroll
+            for (int nib = 0; nib < 2; ++nib) {
+              const __nv_bfloat162 a2 = __float2bfloat162_rn(d * (float)((sc >> (8 * nib)) & 0xffu));
+              const __nv_bfloat162 b2 = __float2bfloat162_rn(-(dmin * (float)((mn >> (8 * nib)) & 0xffu)));
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {                // as unpack_q4k_sub: bf16(16 + q) = 0x4180 | (q << 3)
+                const uint32_t n3 = ((nib ? (w[i] >> 1) : (w[i] << 3)) & 0x78787878u) | 0x80808080u;
+                const uint32_t p0 = prmt(n3, 0x41414141u, 0x4140), p1 = prmt(n3, 0x41414141u, 0x4342);
+                const __nv_bfloat162 x0 = __hfma2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&p0), sixteen), a2, b2);
+                const __nv_bfloat162 x1 = __hfma2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&p1), sixteen), a2, b2);
+                o[16 * nib + 2 * i] = *reinterpret_cast<const uint32_t*>(&x0); o[16 * nib + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&x1);
+              }
+            }
+          } else {
+            const uint4* qp = reinterpret_cast<const uint4*>(rb + row * 272 + 64 * j);
+            const uint32_t scw = *reinterpret_cast<const uint32_t*>(rb + row * 272 + 256 + 4 * j);
+            const __half2 dd = *reinterpret_cast<const __half2*>(&scw);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const float d = v < 2 ? __low2float(dd) : __high2float(dd);
+              const uint4 x4 = qp[v];
+              const uint32_t w[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t x = w[i];
+                const float f0 = (float)(int)(int8_t)(x & 0xff), f1 = (float)(int)(int8_t)((x >> 8) & 0xff);
+                const float f2 = (float)(int)(int8_t)((x >> 16) & 0xff), f3 = (float)(int)(int8_t)(x >> 24);
+                o[8 * v + 2 * i] = pack_bf16x2(f0 * d, f1 * d); o[8 * v + 2 * i + 1] = pack_bf16x2(f2 * d, f3 * d);
+              }
+            }
+          }
+        }
+        __syncwarp();                                      // the raw tile's bytes are in registers
+        if (lane == 0) mbar_arrive(&raw_empty[rs]);
+        if (++rs == RS) { rs = 0; rph ^= 1; }
+        const int first = as;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[as], aph ^ 1, abort_flag, args.status, 1271, as))) { ok = false; break; }
+          tc_fence_after();
+          tmem_st_x32(ta + as * 64, oo[h]);
+          if (++as == kQwA) { as = 0; aph ^= 1; }
+        }
+        if (!ok) break;
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(&a_full[first]); mbar_arrive(&a_full[first + 1]); }       // kQwA is even: a tile's two stages are neighbours
+      }
+    }
+  }
+
+  if (*abort_flag) {                                       // copies may still be landing: bounded grace period
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+}
+
+// Tokens of a tile of the wide kernel: the even cut of the tokens whose rounds of CTAs cost least.  A step of 128 k-columns costs about 170 cycles plus four
+// per token (512 tokens over 40 row tiles: three tiles of 176 tokens in one round, not two of 256 on half of the SMs).
+static int qgemm_wide_tn(int m, int row_tiles, int splits, int sms) {
+  int best = 256;
+  long best_cost = -1;
+  for (int tiles = (m + 255) / 256; tiles <= (m + 63) / 64; ++tiles) {
+    const int tn = ((m + tiles - 1) / tiles + 15) & ~15;
+    const long ctas = (long)row_tiles * ((m + tn - 1) / tn) * splits;
+    const long cost = (ctas + sms - 1) / sms * (170 + 4 * tn);
+    if (best_cost < 0 || cost < best_cost) { best = tn; best_cost = cost; }
+  }
+  return best;
+}
+
+template <int TYPE>
+static int launch_qgemm_wide(const CUtensorMap& tmX, const QWideArgs& a, cudaStream_t stream) {
+  constexpr int RAW = TYPE == 0 ? 128 * 144 : 128 * 272;
+  const int smem = 1024 + qw_b_stages(TYPE) * 32768 + qw_raw_stages(TYPE) * ((RAW + 1023) & ~1023) + 512;
+  auto kern = qgemm_wide_kernel<TYPE>;
+  static bool attr_set = false;
+  if (!attr_set) { GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr_set = true; }
+  int grid = sm_count();
+  const int tiles = a.g.row_tiles * a.g.tok_tiles * a.g.splits;
+  if (tiles < grid) grid = tiles;
+  launch_k(kern, grid, kQwThreads, smem, stream, tmX, a);
+  GB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
 template <int TYPE, int TN>
 static int launch_qgemm(const CUtensorMap& tmX, QGemmArgs a, cudaStream_t stream) {
   constexpr int RAW = TYPE == 0 ? 128 * 144 : 128 * 272;
   constexpr int RAW_PAD = (RAW + 1023) & ~1023;
   constexpr int B_BYTES = TN * 256;
-  // token ring first (2 stages at least, 3 for wide tiles if they fit), the rest of shared memory buys depth for the raw-tile ring:
+  // token ring first, the rest of shared memory buys depth for the raw-tile ring:
   // the quantised bytes in flight are what a decode-sized launch is bound by
   const int budget = 220 * 1024 - 2048 - 2 * kQgA;
-  int bs = TN >= 128 ? 2 : 4;
+  int bs = 4;
   int rs = (budget - bs * B_BYTES) / RAW_PAD;
   if (rs > 4) rs = 4;
-  if (rs >= 3 && TN >= 128 && budget - 3 * B_BYTES >= 2 * RAW_PAD) { bs = 3; rs = (budget - bs * B_BYTES) / RAW_PAD; if (rs > 4) rs = 4; }
   if (rs < 2) return fail("qgemm: token tile does not fit shared memory%s");
   a.b_stages = bs; a.raw_stages = rs;
   const int smem = 1024 + rs * RAW_PAD + 2 * kQgA + bs * B_BYTES + 512;
@@ -315,7 +622,7 @@ static int launch_qgemm(const CUtensorMap& tmX, QGemmArgs a, cudaStream_t stream
 using namespace gb;
 
 // w: tiled Q4_K (ggml type 12) or Q8_0 (8) weights, ceil(n_out / 128) row tiles x k / 256 K tiles.  x bf16 [m, ldx].
-// out bf16 (or f32) [m, ldo].  tn: token tile 16, 32, 64 or 128.  splits > 1 cuts K: `out` is then f32 [splits][m, ldo] (slabs
+// out bf16 (or f32) [m, ldo].  tn: token tile 16, 32, 64, or 128 for more than 64 tokens (the kernel then cuts them itself, into tiles of up to 256).  splits > 1 cuts K: `out` is then f32 [splits][m, ldo] (slabs
 // m * ldo apart), one partial sum per split for the consumer to add; no split may be empty.
 GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* out, int ldo, int out_f32, const float* bias, int n_out,
                     int k, int m, int tn, int splits, void* status, cudaStream_t stream) {
@@ -323,6 +630,9 @@ GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* 
   if (k <= 0 || k % 256 || n_out <= 0) return fail("qgemm: k must be a positive multiple of 256%s");
   if (m <= 0) return 0;
   if (ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return fail("qgemm: operands must be 16-byte aligned%s");
+  if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return fail("qgemm: token tile must be 16, 32, 64 or 128%s");
+  const bool wide = tn == 128;
+  if (wide) tn = qgemm_wide_tn(m, (n_out + 127) / 128, splits > 1 ? splits : 1, sm_count());
   CUtensorMap tmX;
   if (make_tmap_2d(&tmX, x, TM_BF16, (uint64_t)k, (uint64_t)m, (uint64_t)ldx * 2, 64, (uint32_t)tn, TM_SW_128)) return -1;
   QGemmArgs a;
@@ -337,9 +647,13 @@ GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* 
     a.partial_stride = (long)m * ldo;
   }
   const int t = ggml_type == 12 ? 0 : 1;
+  if (wide) {
+    const QWideArgs wa = {a, tn};
+    return t == 0 ? launch_qgemm_wide<0>(tmX, wa, stream) : launch_qgemm_wide<1>(tmX, wa, stream);
+  }
 #define GB_QG(TNV)                                                             \
   if (tn == TNV) return t == 0 ? launch_qgemm<0, TNV>(tmX, a, stream) : launch_qgemm<1, TNV>(tmX, a, stream);
-  GB_QG(16) GB_QG(32) GB_QG(64) GB_QG(128)
+  GB_QG(16) GB_QG(32) GB_QG(64)
 #undef GB_QG
-  return fail("qgemm: token tile must be 16, 32, 64 or 128%s");
+  return fail("qgemm: unsupported token tile%s");
 }

@@ -48,6 +48,22 @@ def test_gemm_matches_fp32_reference(t, rows, k, m):
 
 
 @pytest.mark.parametrize("t", [gt.Q4_K, gt.Q8_0])
+@pytest.mark.parametrize("rows,k,m", [(128, 256, 65), (200, 512, 80), (5120, 512, 129), (384, 2048, 256), (640, 768, 257), (5120, 1024, 512), (19072, 256, 300), (256, 5120, 1025)])
+def test_gemm_wide_tiles(t, rows, k, m):
+    """More than 64 tokens: the operand goes through TMEM, token tiles of 16 to 256.  Edges of tiles, one to many tiles per CTA, rings that wrap."""
+    qw, x, ref = _case(t, rows, k, m, seed=rows + m)
+    bias = torch.randn(rows, device="cuda")
+    out = torch.full((m + 1, rows), 7.0, dtype=torch.bfloat16, device="cuda")
+    qlinear.gemm(x, qw, bias=bias, out=out[:m])
+    f32 = qlinear.gemm(x, qw, bias=bias, out_dtype=torch.float32)
+    _native.assert_status_ok()
+    assert (out[m] == 7).all()
+    assert torch.equal(out[:m], f32.bfloat16())                   # the same sums, rounded
+    assert _rel(f32, ref + bias) < 6e-3                           # weights reach the tensor core rounded to bf16
+    assert (f32 - ref - bias).abs().max() < 0.1 * ref.std()
+
+
+@pytest.mark.parametrize("t", [gt.Q4_K, gt.Q8_0])
 @pytest.mark.parametrize("rows,k,m,splits", [(256, 4096, 8, 2), (640, 8192, 24, 3), (128, 2048, 64, 8), (384, 2560, 5, 4)])
 def test_gemm_k_split_partials_add_up(t, rows, k, m, splits):
     """The K-split form: every split writes its own fp32 slab (bias in the first only); their sum is the plain result."""
