@@ -57,7 +57,13 @@ struct RmsBcast {
 
 // One CTA per row.  Optional: residual[row] += delta[row] first (the sum is written back and is the
 // normalised input); optional MXFP8 output (e4m3 bytes + scale atoms) beside / instead of bf16.
-template <int VPT>   // 8-element vectors per thread (hidden <= 256 * 8 * VPT)
+// A decode step's row is bound by latency: the weights are requested before the dependency wait (no kernel of a step writes them), and the K-split partial
+// sums or the experts' rows of all the thread's vectors in groups of independent loads, added in their order.  Against one load after another: a row of 5120
+// behind seven partials 7.2 -> 3.8 us, 32 rows of 4096 behind four 4.8 -> 2.9 us; 16384 rows of 2048 behind their experts' rows 180 -> 133 us, behind one
+// row each 66 -> 51 us (5.3 TB/s).
+// VPT: 8-element vectors per thread (hidden <= 256 * 8 * VPT).  SRC, what joins the residual: 0 = nothing or bf16 rows, 1 = partial sums, 2 = the experts' rows (an
+// instance each: the loads in flight cost registers, and a prefill's rows want many CTAs per SM instead; as one kernel the 66 us became 102).
+template <int VPT, int SRC>
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ delta, const __nv_bfloat16* __restrict__ x_in,
                const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out, uint8_t* __restrict__ out_q,
@@ -65,13 +71,17 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __rest
                const float* __restrict__ partials, int n_partials, long partial_stride, const uint32_t* wait_flags, int wait_n,
                const uint32_t* epoch_ptr, KernelStatus* st, const __nv_bfloat16* __restrict__ comb_y, const int* __restrict__ comb_rows,
                const float* __restrict__ comb_w, int comb_k, int comb_ld, int part_inner, long part_inner_stride, const RmsBcast bc) {
-  pdl_wait();
-  pdl_trigger();
   const int row = blockIdx.x;
   const int nvec = hidden >> 3;
+  bf16x8 wv[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (threadIdx.x + i * 256 < nvec) wv[i] = *reinterpret_cast<const bf16x8*>(weight + (threadIdx.x + i * 256) * 8);
+  pdl_wait();
+  pdl_trigger();
   __shared__ int c_rows[16];
   __shared__ float c_w[16];
-  if (comb_y != nullptr) {
+  if (SRC == 2) {
     // MoE combine fused into its consumer: delta[row] = sum_j w[row, j] * y[pair_row[row, j]]
     if (threadIdx.x < comb_k) {
       c_rows[threadIdx.x] = comb_rows[(size_t)row * comb_k + threadIdx.x];
@@ -93,66 +103,115 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __rest
       return;
     }
   }
-  if (comb_y != nullptr) __syncthreads();
+  if (SRC == 2) __syncthreads();
   float v[VPT][8];
   float ss = 0.f;
+  auto spread = [](const bf16x8& r, float* f) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { const float2 t = __bfloat1622float2(r.v[u]); f[2 * u] = t.x; f[2 * u + 1] = t.y; }
+  };
+  const __nv_bfloat16* base = residual != nullptr ? residual : x_in;
+  bf16x8 raw[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (threadIdx.x + i * 256 < nvec) raw[i] = *reinterpret_cast<const bf16x8*>(base + (size_t)row * ld_in + (threadIdx.x + i * 256) * 8);
+  const bool plain = SRC == 0 && residual != nullptr && delta != nullptr;
+  float d[VPT][8];                          // what joins the residual
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) d[i][j] = 0.f;
+  if (SRC == 1 && bc.partials_bf16) {
+    // a reduce-scatter that travelled as bf16 rows (prefill-sized tensor parallelism)
+    for (int p = 0; p < n_partials; ++p)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int vi = threadIdx.x + i * 256;
+        if (vi >= nvec) continue;
+        float t8[8];
+        load8(reinterpret_cast<const __nv_bfloat16*>(partials) + (size_t)p * partial_stride + (size_t)row * hidden + vi * 8, t8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[i][j] += t8[j];
+      }
+  } else if (SRC == 1) {
+    // all-reduce fused into its consumer: sum the ranks' fp32 partials in rank order (bit-identical everywhere)
+    // partial p = (rank, K split): ranks are partial_stride apart, the splits of one rank part_inner_stride
+    constexpr int PB = VPT == 1 ? 8 : VPT == 2 ? 4 : 2;
+    const float* src = partials + (size_t)row * hidden;
+    int inner = 0;
+    for (int p0 = 0; p0 < n_partials; p0 += PB) {
+      float4 a[PB][VPT], b[PB][VPT];
+#pragma unroll
+      for (int u = 0; u < PB; ++u) {
+        if (p0 + u < n_partials) {
+#pragma unroll
+          for (int i = 0; i < VPT; ++i)
+            if (threadIdx.x + i * 256 < nvec) {
+              const float4* q = reinterpret_cast<const float4*>(src + (threadIdx.x + i * 256) * 8);
+              a[u][i] = q[0]; b[u][i] = q[1];
+            }
+          if (++inner == part_inner) { inner = 0; src += partial_stride - (long)(part_inner - 1) * part_inner_stride; } else src += part_inner_stride;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < PB; ++u)
+        if (p0 + u < n_partials) {
+#pragma unroll
+          for (int i = 0; i < VPT; ++i) {
+            d[i][0] += a[u][i].x; d[i][1] += a[u][i].y; d[i][2] += a[u][i].z; d[i][3] += a[u][i].w;
+            d[i][4] += b[u][i].x; d[i][5] += b[u][i].y; d[i][6] += b[u][i].z; d[i][7] += b[u][i].w;
+          }
+        }
+    }
+  } else if (SRC == 2) {
+    constexpr int CB = VPT == 1 ? 4 : 2;
+    for (int c0 = 0; c0 < comb_k; c0 += CB) {
+      bf16x8 y[CB][VPT];
+      int rows[CB];
+#pragma unroll
+      for (int u = 0; u < CB; ++u) {
+        rows[u] = c0 + u < comb_k ? c_rows[c0 + u] : -1;
+        if (rows[u] >= 0) {
+#pragma unroll
+          for (int i = 0; i < VPT; ++i)
+            if (threadIdx.x + i * 256 < nvec) y[u][i] = *reinterpret_cast<const bf16x8*>(comb_y + (size_t)rows[u] * comb_ld + (threadIdx.x + i * 256) * 8);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < CB; ++u)
+        if (rows[u] >= 0) {
+          const float w = c_w[c0 + u];
+#pragma unroll
+          for (int i = 0; i < VPT; ++i) {
+            float yv[8];
+            spread(y[u][i], yv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d[i][j] += w * yv[j];
+          }
+        }
+    }
+    // same roundings as the unfused pair of kernels: the combined row is bf16, then the residual sum is bf16
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) d[i][j] = __bfloat162float(__float2bfloat16(d[i][j]));
+  } else if (plain) {
+    bf16x8 dv[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+      if (threadIdx.x + i * 256 < nvec) dv[i] = *reinterpret_cast<const bf16x8*>(delta + (size_t)row * ld_in + (threadIdx.x + i * 256) * 8);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) spread(dv[i], d[i]);
+  }
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int vi = threadIdx.x + i * 256;
     if (vi < nvec) {
-      if (residual != nullptr) {
-        float r[8], d[8];
-        load8(residual + (size_t)row * ld_in + vi * 8, r);
-        if (partials != nullptr) {
-          // all-reduce fused into its consumer: sum the ranks' fp32 partials in rank order (bit-identical everywhere)
+      spread(raw[i], v[i]);
+      if (SRC != 0 || plain) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) d[j] = 0.f;
-          // partial p = (rank, K split): ranks are partial_stride apart, the splits of one rank part_inner_stride
-          if (bc.partials_bf16) {
-            // a reduce-scatter that travelled as bf16 rows (prefill-sized tensor parallelism)
-            for (int p = 0; p < n_partials; ++p) {
-              float t8[8];
-              load8(reinterpret_cast<const __nv_bfloat16*>(partials) + (size_t)p * partial_stride + (size_t)row * hidden + vi * 8, t8);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) d[j] += t8[j];
-            }
-          } else {
-            for (int p = 0; p < n_partials; ++p) {
-              const int po = p / part_inner, pi = p - po * part_inner;
-              const float4* src = reinterpret_cast<const float4*>(partials + (size_t)po * partial_stride + (size_t)pi * part_inner_stride +
-                                                                  (size_t)row * hidden + vi * 8);
-              const float4 a = src[0], b = src[1];
-              d[0] += a.x; d[1] += a.y; d[2] += a.z; d[3] += a.w; d[4] += b.x; d[5] += b.y; d[6] += b.z; d[7] += b.w;
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) r[j] = __bfloat162float(__float2bfloat16(r[j] + d[j]));
-          store8(residual + (size_t)row * ld_in + vi * 8, r);
-        } else if (comb_y != nullptr) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) d[j] = 0.f;
-          for (int c = 0; c < comb_k; ++c) {
-            const int cr = c_rows[c];
-            if (cr < 0) continue;
-            float yv[8];
-            load8(comb_y + (size_t)cr * comb_ld + vi * 8, yv);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) d[j] += c_w[c] * yv[j];
-          }
-          // same roundings as the unfused pair of kernels: the combined row is bf16, then the residual sum is bf16
-#pragma unroll
-          for (int j = 0; j < 8; ++j) r[j] = __bfloat162float(__float2bfloat16(r[j] + __bfloat162float(__float2bfloat16(d[j]))));
-          store8(residual + (size_t)row * ld_in + vi * 8, r);
-        } else if (delta != nullptr) {
-          load8(delta + (size_t)row * ld_in + vi * 8, d);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) r[j] = __bfloat162float(__float2bfloat16(r[j] + d[j]));
-          store8(residual + (size_t)row * ld_in + vi * 8, r);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] = r[j];
-      } else {
-        load8(x_in + (size_t)row * ld_in + vi * 8, v[i]);
+        for (int j = 0; j < 8; ++j) v[i][j] = __bfloat162float(__float2bfloat16(v[i][j] + d[i][j]));
+        store8(residual + (size_t)row * ld_in + vi * 8, v[i]);
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
@@ -172,7 +231,7 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __rest
     float w[8], y[8];
     float amax = 0.f;
     if (vi < nvec) {
-      load8(weight + vi * 8, w);
+      spread(wv[i], w);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         y[j] = __bfloat162float(__float2bfloat16(v[i][j] * scale * w[j]));
@@ -322,6 +381,9 @@ qk_norm_rope_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict
 // The same for head_dim 128 with full rotary (the Qwen3 shape), 16 lanes per (token, head): lane l holds elements 4l..4l+3 and
 // 64+4l..64+4l+3, i.e. both halves of four NeoX pairs, so that every access is an 8-byte vector and a warp moves 256
 // contiguous bytes per instruction (the generic kernel moves 2 bytes per lane).
+// PART: the projection comes as K-split partial sums (an instance of its own: the loads in flight cost registers that a prefill's warps need; without the
+// sums' branch 8143 tokens of 48 heads take 62 us instead of 73).
+template <bool PART>
 __global__ void __launch_bounds__(256)
 qk_norm_rope128_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ slots,
                        const __nv_bfloat16* __restrict__ q_w, const __nv_bfloat16* __restrict__ k_w, __nv_bfloat16* __restrict__ q_out,
@@ -346,14 +408,21 @@ qk_norm_rope128_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restr
     f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
   };
   float xa[4], xb[4];
-  if (part != nullptr) {
+  if constexpr (PART) {
     // the projection arrives as K-split fp32 partial sums [n_part][n_tok][ld_qkv]: summed here in split order
 #pragma unroll
     for (int i = 0; i < 4; ++i) { xa[i] = 0.f; xb[i] = 0.f; }
     const float* pp = part + (size_t)t * ld_qkv + (size_t)h * D + 4 * l;
-    for (int p = 0; p < n_part; ++p, pp += part_stride) {
-      const float4 a = *reinterpret_cast<const float4*>(pp), b = *reinterpret_cast<const float4*>(pp + PAIRS);
-      xa[0] += a.x; xa[1] += a.y; xa[2] += a.z; xa[3] += a.w; xb[0] += b.x; xb[1] += b.y; xb[2] += b.z; xb[3] += b.w;
+    for (int s0 = 0; s0 < n_part; s0 += 4, pp += 4 * part_stride) {            // four at a time in flight
+      float4 a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s0 + u < n_part) { a[u] = *reinterpret_cast<const float4*>(pp + u * part_stride); b[u] = *reinterpret_cast<const float4*>(pp + u * part_stride + PAIRS); }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s0 + u < n_part) {
+          xa[0] += a[u].x; xa[1] += a[u].y; xa[2] += a[u].z; xa[3] += a[u].w; xb[0] += b[u].x; xb[1] += b[u].y; xb[2] += b[u].z; xb[3] += b[u].w;
+        }
     }
   } else {
     unpack4(*reinterpret_cast<const uint2*>(src + 4 * l), xa);
@@ -816,12 +885,15 @@ static int rmsnorm_launch(void* residual, const void* delta, const void* x_in, c
   if (out_q != nullptr && hidden % 128) return fail("rmsnorm: MXFP8 output needs hidden %% 128 == 0%s");
   if (rows <= 0) return 0;
   const int nvec = hidden / 8;
-#define GB_RMS(V) launch_k(rmsnorm_kernel<V>, rows, 256, 0, stream, (__nv_bfloat16*)residual, (const __nv_bfloat16*)delta, \
+  const int src = residual != nullptr && partials != nullptr ? 1 : residual != nullptr && comb_y != nullptr ? 2 : 0;
+#define GB_RMS1(V, S) launch_k(rmsnorm_kernel<V, S>, rows, 256, 0, stream, (__nv_bfloat16*)residual, (const __nv_bfloat16*)delta, \
     (const __nv_bfloat16*)x_in, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out, (uint8_t*)out_q, (uint8_t*)out_sf, hidden, eps, ld_in, ld_out, sf32, \
     partials, n_partials, partial_stride, (const uint32_t*)wait_flags, wait_n, (const uint32_t*)epoch_ptr, (KernelStatus*)status, \
     (const __nv_bfloat16*)comb_y, comb_rows, comb_w, comb_k, comb_ld, part_inner, part_inner_stride, bc)
+#define GB_RMS(V) do { if (src == 1) GB_RMS1(V, 1); else if (src == 2) GB_RMS1(V, 2); else GB_RMS1(V, 0); } while (0)
   if (nvec <= 256) GB_RMS(1); else if (nvec <= 512) GB_RMS(2); else if (nvec <= 768) GB_RMS(3); else GB_RMS(4);
 #undef GB_RMS
+#undef GB_RMS1
   GB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -904,7 +976,7 @@ GB_API int gb_qk_norm_rope_partials(const float* part, int n_part, long part_str
       !al(k_cache, 8) || !al(v_cache, 8) || !al(rope_tab, 16))
     return fail("qk_norm_rope_partials: misaligned argument%s");
   const long warps = (long)n_tok * (hq + 2 * hkv);
-  launch_k(qk_norm_rope128_kernel, (unsigned)((warps + 15) / 16), 256, 0, stream, (const __nv_bfloat16*)nullptr, positions, slots,
+  launch_k(qk_norm_rope128_kernel<true>, (unsigned)((warps + 15) / 16), 256, 0, stream, (const __nv_bfloat16*)nullptr, positions, slots,
            (const __nv_bfloat16*)q_w, (const __nv_bfloat16*)k_w, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache,
            n_tok, hq, hkv, theta, eps, ld_qkv, q_scale, (const float2*)rope_tab, tab_len, pos3, sec_h3, sec_w3, part, n_part, part_stride);
   GB_CUDA_OK(cudaGetLastError());
@@ -920,7 +992,7 @@ GB_API int gb_qk_norm_rope(const void* qkv, const int* positions, const int* slo
   const auto al8 = [](const void* p) { return ((uintptr_t)p & 7) == 0; };
   if (head_dim == 128 && rope_pairs == 64 && ld_qkv % 4 == 0 && al8(qkv) && al8(q_w) && al8(k_w) && al8(q_out) && al8(k_cache) &&
       al8(v_cache) && ((uintptr_t)rope_tab & 15) == 0) {
-    launch_k(qk_norm_rope128_kernel, (unsigned)((warps + 15) / 16), 256, 0, stream, (const __nv_bfloat16*)qkv, positions, slots,
+    launch_k(qk_norm_rope128_kernel<false>, (unsigned)((warps + 15) / 16), 256, 0, stream, (const __nv_bfloat16*)qkv, positions, slots,
              (const __nv_bfloat16*)q_w, (const __nv_bfloat16*)k_w, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache,
              n_tok, hq, hkv, theta, eps, ld_qkv, q_scale, (const float2*)rope_tab, tab_len, pos3, sec_h3, sec_w3, (const float*)nullptr, 0, 0L);
     GB_CUDA_OK(cudaGetLastError());
