@@ -107,13 +107,31 @@ def loaded_libraries():
     return out
 
 
+_raw_stream = _device = None
+
+
+def _bind_torch():
+    global _raw_stream, _device
+    from torch._C import _cuda_getCurrentRawStream, _cuda_getDevice
+    _raw_stream, _device = _cuda_getCurrentRawStream, _cuda_getDevice
+
+
+def stream() -> int:
+    """Handle of torch's current stream on the current device.  (``torch.cuda.current_stream`` makes a Stream object and looks the device up through the
+    environment: 6 us, on every launch.)"""
+    if _device is None:
+        _bind_torch()
+    return _raw_stream(_device())
+
+
 _status_ptrs = {}
 
 
 def status_ptr() -> int:
     """Device address of the status word of the current device (bounded waits report into it)."""
-    import torch
-    dev = torch.cuda.current_device()
+    if _device is None:
+        _bind_torch()
+    dev = _device()
     if dev not in _status_ptrs:
         p = cuda().gb_status_ptr()
         if not p:

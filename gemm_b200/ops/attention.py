@@ -70,7 +70,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cu_
         else:
             part_o = torch.empty(num_splits, t, hq, d, dtype=torch.float32, device=q.device)
             part_lse = torch.empty(num_splits, t, hq, dtype=torch.float32, device=q.device)
-    stream = _c(torch.cuda.current_stream().cuda_stream)
+    stream = _c(_native.stream())
     if decode and USE_DECODE_KERNEL and hq // hkv <= 16:
         rc = lib.gb_flash_decode(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(part_o), _p(part_lse), _p(work), _i(work.shape[0]),
                                  _p(cu_q), _p(kv_len), _p(block_table), _i(block_table.shape[1]), _i(page_size),
@@ -106,7 +106,7 @@ def kv_store_q8(k_src: torch.Tensor, v_src: torch.Tensor, src_slots: Optional[to
         return
     rc = _native.cuda().gb_kv_store_q8(_p(k_src), _p(v_src), _p(src_slots), _p(dst_slots), _p(kq), _p(vq), _p(ks), _p(vs), _i(n),
                                        _i(kq.shape[1]), _i(kq.shape[2]), _l(k_src.shape[0]), _l(kq.shape[0]),
-                                       _c(torch.cuda.current_stream().cuda_stream))
+                                       _c(_native.stream()))
     _native.check(rc, "gb_kv_store_q8")
 
 
@@ -127,7 +127,7 @@ def attention_decode_q8(q: torch.Tensor, kq: torch.Tensor, vq: torch.Tensor, ks:
         part_o = torch.empty(num_splits, b, hq, d, dtype=torch.float32, device=q.device)
         part_lse = torch.empty(num_splits, b, hq, dtype=torch.float32, device=q.device)
     lib = _native.cuda()
-    stream = _c(torch.cuda.current_stream().cuda_stream)
+    stream = _c(_native.stream())
     rc = lib.gb_attn_decode_q8(_p(q), _p(kq), _p(vq), _p(ks), _p(vs), _p(out), _p(part_o), _p(part_lse), _p(kv_len), _p(block_table),
                                _i(block_table.shape[1]), _i(page_size), _l(kq.shape[0]), _i(b), _i(hq), _i(hkv), _i(d), _i(num_splits),
                                _i(window), _c(_native.status_ptr()), stream)
@@ -152,7 +152,7 @@ def attention_decode_mx(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.T
     sf = ew.sf_alloc(rp, hq * d, q.device, sf_layout, init=False)
     if num_splits > 1:
         # split KV ranges: fp32 partials from the decode kernel, merged (and quantised) by the combine kernel
-        lib, stream = _native.cuda(), _c(torch.cuda.current_stream().cuda_stream)
+        lib, stream = _native.cuda(), _c(_native.stream())
         part_o = torch.empty(num_splits, t, hq, d, dtype=torch.float32, device=q.device)
         part_lse = torch.empty(num_splits, t, hq, dtype=torch.float32, device=q.device)
         rc = lib.gb_flash_decode(_p(q), _p(k_cache), _p(v_cache), _c(0), _p(part_o), _p(part_lse), _p(work), _i(work.shape[0]),
@@ -166,7 +166,7 @@ def attention_decode_mx(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.T
     rc = _native.cuda().gb_flash_decode_mx(_p(q), _p(k_cache), _p(v_cache), _p(oq), _p(sf), _i(1 if sf_layout == 32 else 0), _p(work),
                                            _i(work.shape[0]), _p(cu_q), _p(kv_len), _p(block_table), _i(block_table.shape[1]), _i(page_size),
                                            _l(k_cache.shape[0]), _i(t), _i(hq), _i(hkv), _i(d), _i(window), _c(_native.status_ptr()),
-                                           _c(torch.cuda.current_stream().cuda_stream))
+                                           _c(_native.stream()))
     _native.check(rc, "gb_flash_decode_mx")
     return MxTensor(oq, sf, t, hq * d, sf_layout)
 
@@ -185,7 +185,7 @@ def attention_mx(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     rc = _native.cuda().gb_flash_attn_mx(_p(q), _p(k_cache), _p(v_cache), _p(oq), _p(sf), _i(1 if sf_layout == 32 else 0), _p(work),
                                          _i(work.shape[0]), _p(cu_q), _p(kv_len), _p(block_table), _i(block_table.shape[1]), _i(page_size),
                                          _l(k_cache.shape[0]), _i(t), _i(hq), _i(hkv), _i(d), _i(1 if causal else 0), _i(window),
-                                         _c(_native.status_ptr()), _c(torch.cuda.current_stream().cuda_stream))
+                                         _c(_native.status_ptr()), _c(_native.stream()))
     _native.check(rc, "gb_flash_attn_mx")
     return MxTensor(oq, sf, t, hq * d, sf_layout)
 
@@ -218,13 +218,13 @@ def attention_partial(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         rc = _native.cuda().gb_flash_decode(_p(q), _p(k_cache), _p(v_cache), _c(0), _p(part_o), _p(part_lse), _p(work), _i(work.shape[0]),
                                             _p(cu_q), _p(kv_len), _p(block_table), _i(block_table.shape[1]), _i(page_size),
                                             _l(k_cache.shape[0]), _i(t), _i(hq), _i(k_cache.shape[1]), _i(d), _i(num_splits), _i(window),
-                                            _c(_native.status_ptr()), _c(torch.cuda.current_stream().cuda_stream))
+                                            _c(_native.status_ptr()), _c(_native.stream()))
         _native.check(rc, "gb_flash_decode")
         return part_o, part_lse
     rc = _native.cuda().gb_flash_attn(_p(q), _p(k_cache), _p(v_cache), _c(0), _p(part_o), _p(part_lse), _p(work), _i(work.shape[0]),
                                       _p(cu_q), _p(kv_len), _p(block_table), _i(block_table.shape[1]), _i(page_size),
                                       _l(k_cache.shape[0]), _i(t), _i(hq), _i(k_cache.shape[1]), _i(d), _i(num_splits), _i(1 if causal else 0),
-                                      _i(window), _c(_native.status_ptr()), _c(torch.cuda.current_stream().cuda_stream))
+                                      _i(window), _c(_native.status_ptr()), _c(_native.stream()))
     _native.check(rc, "gb_flash_attn")
     return part_o, part_lse
 
@@ -271,7 +271,7 @@ def combine_partials(part_o: torch.Tensor, part_lse: torch.Tensor):
     out = torch.empty(r, d, dtype=torch.bfloat16, device=part_o.device)
     lse = torch.empty(r, dtype=torch.float32, device=part_o.device)
     rc = _native.cuda().gb_fa_combine(_p(part_o), _p(part_lse), _p(out), _p(lse), _i(s), _l(r),
-                                      _c(torch.cuda.current_stream().cuda_stream))
+                                      _c(_native.stream()))
     _native.check(rc, "gb_fa_combine")
     return out, lse
 
@@ -414,7 +414,7 @@ def attention_masked(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         raise ValueError("capped scores and sinks do not go with a distance bias or kept positions")
     out = torch.empty(t, hq, dv, dtype=k_cache.dtype, device=q.device)
     n_bias, ld_bias = (bias.shape[1] // 2, bias.stride(0)) if bias is not None else (0, 0)
-    lib, stream = _native.cuda(), _c(torch.cuda.current_stream().cuda_stream)
+    lib, stream = _native.cuda(), _c(_native.stream())
     if plan is not None and k_cache.dtype == torch.bfloat16 and dk in (64, 128) and dv in (64, 128) and page_size % 8 == 0 and 128 % page_size == 0 \
             and hq // hkv <= 128:
         work, splits = plan

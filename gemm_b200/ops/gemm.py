@@ -7,6 +7,7 @@ no silent fallback on a GPU: a missing library raises).
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -77,8 +78,16 @@ def _p(t: Optional[torch.Tensor]):
     return _c(t.data_ptr()) if t is not None else _c(0)
 
 
+def _at(t: Optional[torch.Tensor]):
+    return t.data_ptr() if t is not None else None
+
+
+def _nbytes(t: Optional[torch.Tensor]) -> int:
+    return t.numel() * t.element_size() if t is not None else 0
+
+
 def _stream():
-    return _c(torch.cuda.current_stream().cuda_stream)
+    return _c(_native.stream())
 
 
 def pick_tn(m_tok: int, mx: bool = False, dual: bool = False) -> int:
@@ -120,12 +129,13 @@ def _launch(w, x, out, n_out, k, m_tok, ldw, ldx, ldo, flags, tn, num_groups=0, 
         extras.wait_flags, extras.wait_n, extras.epoch_ptr = _next_wait
         _next_wait = None
     # extents of the caller's buffers: the kernel checks its scale-atom loads and its stores against them
-    nb = lambda t: t.numel() * t.element_size() if t is not None else 0
-    extras.sfa_bytes, extras.sfb_bytes, extras.out_bytes, extras.out_sf_bytes = nb(sfa), nb(sfb), nb(out), nb(out_sf)
-    rc = lib.gb_gemm(_p(w), _p(x), _p(out), _i(n_out), _i(k), _i(m_tok), _i(ldw), _i(ldx), _i(ldo), _i(flags), _i(tn),
-                     _i(num_groups), _i(w_rows_per_group), _i(up_row_offset), _p(seg_start), _p(seg_count),
-                     _i(x_rows if x_rows is not None else m_tok), _p(sfa), _p(sfb), _p(out_sf), _p(bias), _p(row_map),
-                     _p(row_scale), ctypes.byref(extras) if extras is not None else _c(0), _c(_native.status_ptr()), _stream())
+    extras.sfa_bytes, extras.sfb_bytes, extras.out_bytes, extras.out_sf_bytes = _nbytes(sfa), _nbytes(sfb), _nbytes(out), _nbytes(out_sf)
+    fn = lib.gb_gemm
+    if fn.argtypes is None:            # plain integers from here on: 27 wrapped arguments cost as much as the launch
+        fn.argtypes = [_c] * 3 + [_i] * 11 + [_c] * 2 + [_i] + [_c] * 6 + [ctypes.POINTER(GemmExtras)] + [_c] * 2
+    rc = fn(_at(w), _at(x), _at(out), n_out, k, m_tok, ldw, ldx, ldo, flags, tn, num_groups, w_rows_per_group, up_row_offset, _at(seg_start), _at(seg_count),
+            x_rows if x_rows is not None else m_tok, _at(sfa), _at(sfb), _at(out_sf), _at(bias), _at(row_map), _at(row_scale), extras, _native.status_ptr(),
+            _native.stream())
     if restore is not None:
         extras.wait_flags, extras.wait_n, extras.epoch_ptr = restore
     _native.check(rc, "gb_gemm")
@@ -292,6 +302,7 @@ class PendingPartials:
         return self.buf.sum(0).to(torch.bfloat16)
 
 
+@functools.lru_cache(maxsize=4096)
 def pick_partials(n_out: int, m_tok: int, k: int, mx: bool, sms: int = 148) -> int:
     """Number of K splits for a decode-sized projection: the split count (at most 8, at least 4 k-steps per split, no empty split)
     that fills the last wave of CTAs best; ties go to fewer splits.  96 tiles -> 3 splits (288 CTAs = 1.95 waves), 16 tiles -> 8."""

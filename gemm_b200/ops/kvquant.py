@@ -34,7 +34,7 @@ def quantize_q8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     q = torch.empty(xc.shape, dtype=torch.int8, device=x.device)
     sc = torch.empty(xc.shape[:-1], dtype=torch.float32, device=x.device)
     rc = _native.cuda().gb_kv_quant_q8(_c(xc.data_ptr()), _c(q.data_ptr()), _c(sc.data_ptr()), _l(rows), _i(d),
-                                       _c(torch.cuda.current_stream().cuda_stream))
+                                       _c(_native.stream()))
     _native.check(rc, "gb_kv_quant_q8")
     return q, sc
 
@@ -47,6 +47,6 @@ def dequantize_q8(q: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
     qc, sc = q.contiguous(), scale.contiguous()
     out = torch.empty(qc.shape, dtype=torch.bfloat16, device=q.device)
     rc = _native.cuda().gb_kv_dequant_q8(_c(qc.data_ptr()), _c(sc.data_ptr()), _c(out.data_ptr()), _l(qc.numel() // d), _i(d),
-                                         _c(torch.cuda.current_stream().cuda_stream))
+                                         _c(_native.stream()))
     _native.check(rc, "gb_kv_dequant_q8")
     return out

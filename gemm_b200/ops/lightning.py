@@ -21,7 +21,7 @@ def _p(t):
 
 
 def _s():
-    return _c(torch.cuda.current_stream().cuda_stream)
+    return _c(_native.stream())
 
 
 # Launches whose longest sequence brings at least this many tokens take the chunked scan (csrc/kernels/lightning_chunk.cu): its chain has

@@ -26,7 +26,7 @@ def _p(t):
 
 
 def _s():
-    return _c(torch.cuda.current_stream().cuda_stream)
+    return _c(_native.stream())
 
 
 def router_logits(h: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

@@ -78,7 +78,7 @@ class QGemvPeer(ctypes.Structure):
 
 
 def _stream():
-    return _c(torch.cuda.current_stream().cuda_stream)
+    return _c(_native.stream())
 
 
 def pick_splits(rows: int, k: int, m: int, ggml_type: int = gt.Q4_K, sms: int = 148) -> int:

@@ -54,7 +54,7 @@ class QuantWeight:
         _ensure_codebooks(self.raw.device)
         out = torch.empty(self.rows, self.k, dtype=torch.bfloat16, device=self.raw.device)
         rc = _native.cuda().gb_dequant_bf16(_c(self.raw.data_ptr()), _c(out.data_ptr()), _l(n), _i(self.ggml_type),
-                                            _c(torch.cuda.current_stream().cuda_stream))
+                                            _c(_native.stream()))
         _native.check(rc, "gb_dequant_bf16")
         return out
 
@@ -68,7 +68,7 @@ def linear_quant(x: torch.Tensor, w: QuantWeight, out_dtype=torch.bfloat16) -> t
         _ensure_codebooks(x.device)
         y = torch.empty(m, w.rows, dtype=torch.float32, device=x.device)
         rc = _native.cuda().gb_gemv_quant(_c(w.raw.data_ptr()), _c(x.data_ptr()), _c(y.data_ptr()), _i(w.rows), _i(w.k), _i(m), _i(w.ggml_type),
-                                          _i(x.stride(0)), _i(w.rows), _c(torch.cuda.current_stream().cuda_stream))
+                                          _i(x.stride(0)), _i(w.rows), _c(_native.stream()))
         _native.check(rc, "gb_gemv_quant")
         return y if out_dtype == torch.float32 else y.to(out_dtype)
     from . import gemm

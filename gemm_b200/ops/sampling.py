@@ -31,7 +31,7 @@ def argmax(logits: torch.Tensor, idx_offset: int = 0, want_value: bool = False):
     out = torch.empty(b, dtype=torch.int32, device=logits.device)
     val = torch.empty(b, dtype=torch.float32, device=logits.device) if want_value else None
     dt = 0 if logits.dtype == torch.float32 else 1
-    stream = _c(torch.cuda.current_stream().cuda_stream)
+    stream = _c(_native.stream())
     if v >= 16384:
         chunks = max(1, min(64, 1184 // max(1, b)))
         pv = torch.empty(chunks * b, dtype=torch.float32, device=logits.device)
@@ -58,7 +58,7 @@ def sample(logits: torch.Tensor, temperature: float = 1.0, top_k: int = 0, top_p
     out = torch.empty(b, dtype=torch.int32, device=logits.device)
     dt = 0 if logits.dtype == torch.float32 else 1
     rc = _native.cuda().gb_sample(_p(logits), _p(out), _i(b), _i(v), _l(logits.stride(0)), _i(dt), _f(temperature), _i(top_k),
-                                  _f(top_p), _u64(seed), _u64(step), _p(step_ctr), _c(torch.cuda.current_stream().cuda_stream))
+                                  _f(top_p), _u64(seed), _u64(step), _p(step_ctr), _c(_native.stream()))
     _native.check(rc, "gb_sample")
     return out
 

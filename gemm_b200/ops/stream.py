@@ -39,7 +39,7 @@ def _p(t):
 
 
 def _s():
-    return _c(torch.cuda.current_stream().cuda_stream)
+    return _c(_native.stream())
 
 
 def row_width(n: int, dtype: torch.dtype) -> int:
