@@ -288,10 +288,6 @@ BRANCHES = os.environ.get("GB_BRANCHES", "1") != "0"
 PAIR_DOWN = os.environ.get("GB_PAIR_DOWN", "1") != "0"
 
 
-# steps of one or two tokens on GEMVs with the token-wise work fused in (GB_NARROW=0: the kernels of larger batches)
-NARROW = os.environ.get("GB_NARROW", "1") != "0"
-
-
 class SingleProcess:
     """Parallel context of an unsharded model: every collective is the identity."""
     tp_size = 1
@@ -901,8 +897,6 @@ class Transformer:
             # plain dense stacks (nothing reads the whole stream or the normalised rows outside a GEMM in between)
             self.par._sp_ok = not (cfg.is_moe or cfg.attn_output_gate or fb.deepstack is not None or self.snapshot_layers or
                                    any(l.ssm is not None for l in w.layers[first_layer:last_layer]))
-        if self.narrow_ok(x, fb, first_layer, last_layer):
-            return self.narrow_layers(x, fb, first_layer, last_layer)
         for li in range(first_layer, last_layer):           # li: the layer RUN, index of its cache (looped layers run several times)
             lw = w.layers[self.runs[li].layer]
             if cfg.parallel_ffn:
@@ -968,40 +962,6 @@ class Transformer:
             self._last_delta = delta
             return x
         self._last_delta = self.par.materialize(delta) if delta is not None else None
-        return x
-
-    def narrow_ok(self, x: torch.Tensor, fb: ForwardBatch, first_layer: int, last_layer: int) -> bool:
-        """Whether a step of one or two tokens runs on ``narrow_layers``: dense bf16 layers of one process, nothing that reads the stream in between."""
-        cfg = self.cfg
-        if not (NARROW and x.is_cuda and 1 <= x.shape[0] <= gemm.GEMV_MAX_TOKENS and type(self.par) is SingleProcess and x.dtype == torch.bfloat16 and x.is_contiguous()):
-            return False
-        if self.stream_f32 or self.mx or cfg.is_moe or cfg.attn_output_gate or self.kv.quantized or fb.deepstack is not None or self.snapshot_layers:
-            return False
-        if cfg.hidden > gemm.GEMV_MAX_NORM_K or cfg.hidden % 64 or first_layer == last_layer:
-            return False
-        layers = self.w.layers[first_layer:last_layer]
-        mats = [m for lw in layers for m in (lw.wqkv, lw.wo, lw.w_gate_up, lw.w_down)]
-        return all(m is not None and m.fmt == "bf16" and not m.is_quant and m.k % 64 == 0 and m.w.stride(1) == 1 for m in mats) and \
-            all(lw.w_gate_up.bias is None for lw in layers)
-
-    def narrow_layers(self, x: torch.Tensor, fb: ForwardBatch, first_layer: int, last_layer: int) -> torch.Tensor:
-        """The layers of a step of one or two tokens: every projection is a GEMV whose launch also does the residual add and RMSNorm in front of it, or the
-        activation behind it (six launches a layer instead of nine)."""
-        cfg, delta = self.cfg, None
-        for li in range(first_layer, last_layer):
-            lw = self.w.layers[li]
-            with profiler.region("attention", "block", "attention", li):
-                qkv, x = gemm.gemv_norm(x, delta, lw.attn_norm, cfg.rms_eps, lw.wqkv.w, lw.wqkv.bias, lw.wqkv.tiled)
-                q = ew.qk_norm_rope(qkv, fb.positions, fb.slots, lw.q_norm, lw.k_norm, self.kv.k[li], self.kv.v[li], self.hq_local, self.hkv_local, cfg.head_dim,
-                                    cfg.rope_theta, cfg.rms_eps, self.q_scale, self.rope_dim, table=self.rope_table, positions3=fb.positions3,
-                                    sections=cfg.mrope_sections)
-                a = att.attention(q, self.kv.k[li], self.kv.v[li], fb.cu_q, fb.kv_len, fb.block_table, self.kv.page_size, fb.work, num_splits=fb.num_splits,
-                                  causal=True, window=cfg.sliding_window, decode=fb.is_decode)
-                delta = gemm.gemv(a.reshape(a.shape[0], -1), lw.wo.w, lw.wo.bias, lw.wo.tiled)
-            with profiler.region("ffn", "block", "ffn", li):
-                act, x = gemm.gemv_norm(x, delta, lw.ffn_norm, cfg.rms_eps, lw.w_gate_up.w, w_tiled=lw.w_gate_up.tiled, swiglu=True)
-                delta = gemm.gemv(act, lw.w_down.w, lw.w_down.bias, lw.w_down.tiled)
-        self._last_delta = delta.materialize()
         return x
 
     def forward(self, fb: ForwardBatch) -> torch.Tensor:

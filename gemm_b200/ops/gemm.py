@@ -336,40 +336,6 @@ def linear_partials(x: torch.Tensor, w: torch.Tensor, splits: int, bias: Optiona
     return PendingPartials(out)
 
 
-GEMV_MAX_TOKENS = 2                  # csrc/kernels/gemv.cu
-GEMV_MAX_NORM_K = 8192
-
-
-def _gemv(w, k, n, up, m, x, residual, res_out, delta, norm_w, eps, out, act, bias, w_tiled):
-    rc = _native.cuda().gb_gemv(_p(w), _i(w.stride(0)), _i(1 if w_tiled else 0), _i(n), _i(k), _i(up), _i(m), _p(x), _i(x.stride(0) if x is not None else 0),
-                                _p(residual), _p(res_out), _p(delta.buf if delta is not None else None), _i(delta.n if delta is not None else 0),
-                                ctypes.c_long(m * k), _p(norm_w), ctypes.c_float(eps), _p(out), _p(act), _i(n), _p(bias), _stream())
-    _native.check(rc, "gb_gemv")
-
-
-def gemv(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, w_tiled: bool = False) -> PendingPartials:
-    """bf16 ``linear`` of one or two tokens without tensor cores: f32 sums for the consumer, one slab (GPU only)."""
-    m, k = x.shape
-    n = w.shape[0]
-    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1 and 1 <= m <= GEMV_MAX_TOKENS
-    out = torch.empty(1, m, n, dtype=torch.float32, device=x.device)
-    _gemv(w, k, n, 0, m, x, None, None, None, None, 0.0, out, None, bias, w_tiled)
-    return PendingPartials(out)
-
-
-def gemv_norm(residual: torch.Tensor, delta: Optional[PendingPartials], norm_w: torch.Tensor, eps: float, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
-              w_tiled: bool = False, swiglu: bool = False):
-    """The residual add and RMSNorm in front of ``gemv`` in the same launch: ``(result, new residual)``.  The residual rows ``[m, k]`` are not written to:
-    the sum is a new tensor (they themselves without ``delta``).  ``swiglu``: ``w = [Wg; Wu]``, the result is bf16 ``silu(h Wg^T) * (h Wu^T)`` instead of f32 sums."""
-    m, k = residual.shape
-    assert residual.is_contiguous() and residual.dtype == torch.bfloat16 and w.stride(1) == 1 and 1 <= m <= GEMV_MAX_TOKENS
-    n = w.shape[0] // 2 if swiglu else w.shape[0]
-    res_out = torch.empty_like(residual) if delta is not None else None
-    out = torch.empty(m, n, dtype=torch.bfloat16, device=w.device) if swiglu else torch.empty(1, m, n, dtype=torch.float32, device=w.device)
-    _gemv(w, k, n, n if swiglu else 0, m, None, residual, res_out, delta, norm_w, eps, None if swiglu else out, out if swiglu else None, bias, w_tiled)
-    return (out if swiglu else PendingPartials(out)), (res_out if delta is not None else residual)
-
-
 def pick_partials_dual(inter: int, m_tok: int, k: int, mx: bool) -> int:
     """K splits for a decode-sized gate/up projection (a tile = 128 gate rows + 128 up rows)."""
     return pick_partials(inter, m_tok, k, mx)
