@@ -581,11 +581,21 @@ silu_mul_partials_kernel(const float* __restrict__ part, int n_part, long part_s
 #pragma unroll
     for (int j = 0; j < 8; ++j) { g[j] = bias != nullptr ? bias[vi * 8 + j] : 0.f; u[j] = bias != nullptr ? bias[inter + vi * 8 + j] : 0.f; }
     const float* pp = part + r * (2L * inter) + vi * 8;
-    for (int p = 0; p < n_part; ++p, pp += part_stride) {
-      const float4 g0 = *reinterpret_cast<const float4*>(pp), g1 = *reinterpret_cast<const float4*>(pp + 4);
-      const float4 u0 = *reinterpret_cast<const float4*>(pp + inter), u1 = *reinterpret_cast<const float4*>(pp + inter + 4);
-      g[0] += g0.x; g[1] += g0.y; g[2] += g0.z; g[3] += g0.w; g[4] += g1.x; g[5] += g1.y; g[6] += g1.z; g[7] += g1.w;
-      u[0] += u0.x; u[1] += u0.y; u[2] += u0.z; u[3] += u0.w; u[4] += u1.x; u[5] += u1.y; u[6] += u1.z; u[7] += u1.w;
+    for (int p0 = 0; p0 < n_part; p0 += 4, pp += 4 * part_stride) {            // four slabs' loads in flight
+      float4 x[4][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (p0 + e < n_part) {
+          const float* q = pp + e * part_stride;
+          x[e][0] = *reinterpret_cast<const float4*>(q); x[e][1] = *reinterpret_cast<const float4*>(q + 4);
+          x[e][2] = *reinterpret_cast<const float4*>(q + inter); x[e][3] = *reinterpret_cast<const float4*>(q + inter + 4);
+        }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (p0 + e < n_part) {
+          g[0] += x[e][0].x; g[1] += x[e][0].y; g[2] += x[e][0].z; g[3] += x[e][0].w; g[4] += x[e][1].x; g[5] += x[e][1].y; g[6] += x[e][1].z; g[7] += x[e][1].w;
+          u[0] += x[e][2].x; u[1] += x[e][2].y; u[2] += x[e][2].z; u[3] += x[e][2].w; u[4] += x[e][3].x; u[5] += x[e][3].y; u[6] += x[e][3].z; u[7] += x[e][3].w;
+        }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
