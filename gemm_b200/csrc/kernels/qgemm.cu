@@ -285,19 +285,19 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const QGemmArgs args) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------------------------------
-// More than 64 tokens.  The kernel above is then bound by shared memory: per 128 x 128 step of W it writes 32 KB of unpacked operand, and the MMAs read that and
-// the tokens' 32 KB again, 1470 cycles of the SM's shared memory for 512 of the tensor core, and every 128 tokens unpack W anew.  Here the unpacked operand never
-// meets shared memory: eight warps (a thread per weight row and 64-value chunk) write it straight into TMEM (tcgen05.st) and the MMA takes its A operand from
-// there; the token tile is up to 256 wide, so W is unpacked once per 256 tokens.  Same operands, same order of sums as above.  Qwen3-32B's four projections of
-// 512 tokens: QW_MEASURED.
+// More than 128 tokens.  The kernel above unpacks W anew for every 128 tokens, and writes it to shared memory for the MMAs to read back.  Here the unpacked operand
+// never meets shared memory: sixteen warps (a thread per weight row and 64-value chunk) write it straight into TMEM (tcgen05.st) and the MMA takes its A operand
+// from there; what shared memory keeps free holds token tiles of up to 256, so W is unpacked once per 256 tokens.  Same operands, same order of sums as above.
+// 512 tokens by 51200 rows of 5120: 379 -> 247 us, by 5120 rows of 25600: 334 -> 188 us.
 //
 // TMEM: columns 0-255 accumulators (one of up to 256 columns, or two of up to 128), 256-511 four operand stages of 128 rows x 128 bf16 (64 columns each).
-// Roles (576 threads): warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue (token half (warp - 2) / 4), warps 10-17 unpack (chunk (warp - 10) / 4 of a stage).
-constexpr int kQwThreads = 576;
+// Roles (864 threads): warp 0 producer of token tiles, warp 26 of raw tiles, warp 1 MMA issuer, warps 2-9 epilogue (token half (warp - 2) / 4), warps 10-25
+// unpack: two groups of eight take the raw tiles in turn (one group alone: 5 to 10 % more), and each fills its own two operand stages.
+constexpr int kQwThreads = 864;
 constexpr int kQwA = 4;                    // operand stages in TMEM
 // Stages of 64 token columns (32 KB each) and raw tiles (18 KB Q4_K, 34 KB Q8_0) in flight: what shared memory holds, the tokens' bytes first.
-__host__ __device__ constexpr int qw_b_stages(int type) { return type == 0 ? 5 : 4; }
-__host__ __device__ constexpr int qw_raw_stages(int type) { return type == 0 ? 3 : 2; }
+__host__ __device__ constexpr int qw_b_stages(int type) { return type == 0 ? 4 : 3; }
+__host__ __device__ constexpr int qw_raw_stages(int type) { return type == 0 ? 4 : 3; }
 
 struct QWideArgs {
   QGemmArgs g;
@@ -357,25 +357,35 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
   pdl_trigger();
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ producer
+    // ------------------------------------------------------------------ producer of token tiles
     if (lane == 0) {
-      int rs = 0; uint32_t rph = 0; int bs = 0; uint32_t bph = 0;
+      int bs = 0; uint32_t bph = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
+        int rt, tb, kb0, kb1;
+        tile_at(t, rt, tb, kb0, kb1);
+        for (int h = 4 * kb0; h < 4 * kb1; ++h) {
+          if (!mbar_wait(&b_empty[bs], bph ^ 1, abort_flag, args.status, 1241, bs)) { ok = false; break; }
+          mbar_expect_tx(&b_full[bs], b_bytes);
+          tma_load_2d(Bb + bs * 32768, &tmX, &b_full[bs], h * 64, tb * TN);
+          if (++bs == BS) { bs = 0; bph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 26) {
+    // ------------------------------------------------------------------ producer of raw tiles
+    if (lane == 0) {
+      int rs = 0; uint32_t rph = 0;
       bool ok = true;
       for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
         int rt, tb, kb0, kb1;
         tile_at(t, rt, tb, kb0, kb1);
         const uint8_t* wt = args.w + (size_t)rt * args.num_kb * RAW;
-        for (int kb = kb0; ok && kb < kb1; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&raw_empty[rs], rph ^ 1, abort_flag, args.status, 1240, rs)) { ok = false; break; }
           mbar_expect_tx(&raw_full[rs], RAW);
           bulk_load(rawb + rs * RAW_PAD, wt + (size_t)kb * RAW, RAW, &raw_full[rs]);
           if (++rs == RS) { rs = 0; rph ^= 1; }
-          for (int h = 0; h < 4; ++h) {
-            if (!mbar_wait(&b_empty[bs], bph ^ 1, abort_flag, args.status, 1241, bs)) { ok = false; break; }
-            mbar_expect_tx(&b_full[bs], b_bytes);
-            tma_load_2d(Bb + bs * 32768, &tmX, &b_full[bs], kb * 256 + h * 64, tb * TN);
-            if (++bs == BS) { bs = 0; bph ^= 1; }
-          }
         }
       }
     }
@@ -427,65 +437,47 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
       const float bias = (args.bias != nullptr && n_ok && ksp == 0) ? args.bias[n] : 0.f;
       const int tok0 = tb * TN + c0, live = min(min(128, TN - c0), args.m_tok - tok0);        // this warp's tokens (may be <= 0)
       const size_t off0 = (size_t)ksp * (size_t)args.partial_stride + (size_t)tok0 * args.ldo + n;
-      if (!args.out_f32) {
-        // everything out of TMEM as packed bf16 before the stores: a 256-token tile has no second accumulator to go on with
-        uint32_t pk[64];
-#pragma unroll
-        for (int c = 0; c < 128; c += 16) {
-          if (c < live) {
-            uint32_t r[16];
-            tmem_ld_x16(tacc + c, r);
-            tc_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 8; ++j) pk[c / 2 + j] = pack_bf16x2(__uint_as_float(r[2 * j]) + bias, __uint_as_float(r[2 * j + 1]) + bias);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[acc]);
-        if (n_ok) {
-          unsigned short* o = reinterpret_cast<unsigned short*>(args.out) + off0;
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            if (2 * i < live) o[(size_t)(2 * i) * args.ldo] = (unsigned short)(pk[i] & 0xffffu);
-            if (2 * i + 1 < live) o[(size_t)(2 * i + 1) * args.ldo] = (unsigned short)(pk[i] >> 16);
-          }
-        }
-      } else {
 #pragma unroll 1
-        for (int c = 0; c < live; c += 16) {
-          uint32_t r[16];
-          tmem_ld_x16(tacc + c, r);
-          tc_wait_ld();
-          if (!n_ok) continue;
-          float* o = reinterpret_cast<float*>(args.out) + off0 + (size_t)c * args.ldo;
+      for (int c = 0; c < live; c += 16) {
+        uint32_t r[16];
+        tmem_ld_x16(tacc + c, r);
+        tc_wait_ld();
+        if (!n_ok) continue;
+        const size_t off = off0 + (size_t)c * args.ldo;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) if (c + j < live) o[(size_t)j * args.ldo] = __uint_as_float(r[j]) + bias;
+        for (int j = 0; j < 16; ++j) {
+          if (c + j >= live) break;
+          const float v = __uint_as_float(r[j]) + bias;
+          if (args.out_f32) reinterpret_cast<float*>(args.out)[off + (size_t)j * args.ldo] = v;
+          else reinterpret_cast<__nv_bfloat16*>(args.out)[off + (size_t)j * args.ldo] = __float2bfloat16(v);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[acc]);
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acce[acc]);
       if (++acc == nacc) { acc = 0; acc_ph ^= 1; }
     }
   } else {
-    // ------------------------------------------------------------------ unpack (warps 10..17): raw blocks -> operand in TMEM
-    const int q = warp & 3, part = (warp - 10) >> 2, row = q * 32 + lane;
-    const uint32_t ta = tmem_a + part * 32 + ((uint32_t)(q * 32) << 16);
-    int rs = 0; uint32_t rph = 0; int as = 0; uint32_t aph = 0;
+    // ------------------------------------------------------------------ unpack (warps 10..25): raw blocks -> operand in TMEM
+    const int q = warp & 3, part = ((warp - 10) >> 2) & 1, grp = (warp - 10) >> 3, row = q * 32 + lane;
+    const uint32_t ta = tmem_a + grp * 128 + part * 32 + ((uint32_t)(q * 32) << 16);
+    int rs = 0; uint32_t rph = 0, aph = 0; int turn = 0;
     bool ok = true;
     for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
       int rt, tb, kb0, kb1;
       tile_at(t, rt, tb, kb0, kb1);
-      for (int kb = kb0; ok && kb < kb1; ++kb) {
+      for (int kb = kb0; ok && kb < kb1; ++kb, turn ^= 1) {
+        const int slot = rs;
+        const uint32_t slot_ph = rph;
+        if (++rs == RS) { rs = 0; rph ^= 1; }
+        if (turn != grp) continue;
         // warp-uniform, as are all steps below (stores to TMEM are a warp's)
-        if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rs], rph, abort_flag, args.status, 1270, rs))) { ok = false; break; }
-        const uint8_t* rb = rawb + rs * RAW_PAD;
-        uint32_t oo[2][32];                                // both stages of the tile, two values a word, in k order
+        if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[slot], slot_ph, abort_flag, args.status, 1270, slot))) { ok = false; break; }
+        const uint8_t* rb = rawb + slot * RAW_PAD;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int j = 2 * h + part;                      // 64-value chunk of the 256-column tile
-          uint32_t* o = oo[h];
+          uint32_t o[32];                                  // two values each, in k order
           if (TYPE == 0) {
             const uint8_t* b = rb + row * 144;
             const uint4 hd = *reinterpret_cast<const uint4*>(b);
@@ -532,23 +524,19 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
               }
             }
           }
-        }
-        __syncwarp();                                      // the raw tile's bytes are in registers
-        if (lane == 0) mbar_arrive(&raw_empty[rs]);
-        if (++rs == RS) { rs = 0; rph ^= 1; }
-        const int first = as;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          const int as = 2 * grp + h;
           if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[as], aph ^ 1, abort_flag, args.status, 1271, as))) { ok = false; break; }
           tc_fence_after();
-          tmem_st_x32(ta + as * 64, oo[h]);
-          if (++as == kQwA) { as = 0; aph ^= 1; }
+          tmem_st_x32(ta + h * 64, o);
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&a_full[as]);
+            if (h == 1) mbar_arrive(&raw_empty[slot]);     // the words stored above were formed from the tile's bytes: all reads of it have returned
+          }
         }
-        if (!ok) break;
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&a_full[first]); mbar_arrive(&a_full[first + 1]); }       // kQwA is even: a tile's two stages are neighbours
+        aph ^= 1;
       }
     }
   }
@@ -563,15 +551,15 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-// Tokens of a tile of the wide kernel: the even cut of the tokens whose rounds of CTAs cost least.  A step of 128 k-columns costs about 170 cycles plus four
-// per token (512 tokens over 40 row tiles: three tiles of 176 tokens in one round, not two of 256 on half of the SMs).
+// Tokens of a tile of the wide kernel: the even cut of the tokens whose rounds of CTAs cost least.  A step of 128 k-columns costs much the same for any tile, a
+// little more for a wide one (512 tokens over 40 row tiles: three tiles of 176 tokens in one round).
 static int qgemm_wide_tn(int m, int row_tiles, int splits, int sms) {
   int best = 256;
   long best_cost = -1;
   for (int tiles = (m + 255) / 256; tiles <= (m + 63) / 64; ++tiles) {
     const int tn = ((m + tiles - 1) / tiles + 15) & ~15;
     const long ctas = (long)row_tiles * ((m + tn - 1) / tn) * splits;
-    const long cost = (ctas + sms - 1) / sms * (170 + 4 * tn);
+    const long cost = (ctas + sms - 1) / sms * (600 + 2 * tn);
     if (best_cost < 0 || cost < best_cost) { best = tn; best_cost = cost; }
   }
   return best;
@@ -600,7 +588,7 @@ static int launch_qgemm(const CUtensorMap& tmX, QGemmArgs a, cudaStream_t stream
   // token ring first, the rest of shared memory buys depth for the raw-tile ring:
   // the quantised bytes in flight are what a decode-sized launch is bound by
   const int budget = 220 * 1024 - 2048 - 2 * kQgA;
-  int bs = 4;
+  const int bs = TN < 128 ? 4 : TYPE == 0 ? 3 : 2;
   int rs = (budget - bs * B_BYTES) / RAW_PAD;
   if (rs > 4) rs = 4;
   if (rs < 2) return fail("qgemm: token tile does not fit shared memory%s");
@@ -622,7 +610,7 @@ static int launch_qgemm(const CUtensorMap& tmX, QGemmArgs a, cudaStream_t stream
 using namespace gb;
 
 // w: tiled Q4_K (ggml type 12) or Q8_0 (8) weights, ceil(n_out / 128) row tiles x k / 256 K tiles.  x bf16 [m, ldx].
-// out bf16 (or f32) [m, ldo].  tn: token tile 16, 32, 64, or 128 for more than 64 tokens (the kernel then cuts them itself, into tiles of up to 256).  splits > 1 cuts K: `out` is then f32 [splits][m, ldo] (slabs
+// out bf16 (or f32) [m, ldo].  tn: token tile 16, 32, 64, or 128 for more than 64 tokens (which may then be cut into tiles of up to 256).  splits > 1 cuts K: `out` is then f32 [splits][m, ldo] (slabs
 // m * ldo apart), one partial sum per split for the consumer to add; no split may be empty.
 GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* out, int ldo, int out_f32, const float* bias, int n_out,
                     int k, int m, int tn, int splits, void* status, cudaStream_t stream) {
@@ -631,8 +619,16 @@ GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* 
   if (m <= 0) return 0;
   if (ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return fail("qgemm: operands must be 16-byte aligned%s");
   if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return fail("qgemm: token tile must be 16, 32, 64 or 128%s");
-  const bool wide = tn == 128;
-  if (wide) tn = qgemm_wide_tn(m, (n_out + 127) / 128, splits > 1 ? splits : 1, sm_count());
+  // A step of 128 k-columns takes the wide kernel about a tenth longer than the narrow one, whatever the tile's tokens: it is taken where its wider tiles save
+  // a round of CTAs (51200 rows of 5120: 128 tokens 107 us narrow, 117 wide; 160 tokens 204 and 122; 512 tokens 371 and 247; 5120 rows of 8192: 384 tokens 61
+  // and 65, 512 tokens 114 and 65).
+  bool wide = false;
+  if (tn == 128) {
+    const int row_tiles = (n_out + 127) / 128, sp = splits > 1 ? splits : 1, sms = sm_count(), wtn = qgemm_wide_tn(m, row_tiles, sp, sms);
+    auto rounds = [&](int t) { return ((long)row_tiles * ((m + t - 1) / t) * sp + sms - 1) / sms; };
+    wide = rounds(wtn) < rounds(128);
+    if (wide) tn = wtn;
+  }
   CUtensorMap tmX;
   if (make_tmap_2d(&tmX, x, TM_BF16, (uint64_t)k, (uint64_t)m, (uint64_t)ldx * 2, 64, (uint32_t)tn, TM_SW_128)) return -1;
   QGemmArgs a;
@@ -653,7 +649,7 @@ GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* 
   }
 #define GB_QG(TNV)                                                             \
   if (tn == TNV) return t == 0 ? launch_qgemm<0, TNV>(tmX, a, stream) : launch_qgemm<1, TNV>(tmX, a, stream);
-  GB_QG(16) GB_QG(32) GB_QG(64)
+  GB_QG(16) GB_QG(32) GB_QG(64) GB_QG(128)
 #undef GB_QG
   return fail("qgemm: unsupported token tile%s");
 }
