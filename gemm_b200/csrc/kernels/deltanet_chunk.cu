@@ -11,14 +11,15 @@
 //
 // Two kernels.  dn_chunk_prep_kernel (one CTA per chunk and value head, all chunks of all sequences in parallel) computes what
 // does not depend on the state: the normalised q / k, T (forward substitution, one thread per column), T V, -T diag(exp c) K, M,
-// diag(exp c) Q and the decayed keys, all as bf16 tiles in a workspace.  dn_chunk_scan_kernel (one CTA per sequence and value head)
-// walks the chunks in order: three products per chunk (U, O, the state update), the gated RMSNorm of O, and the output.  The products
+// diag(exp c) Q and the decayed keys, all as bf16 tiles in a workspace.  dn_chunk_scan_kernel (one or two CTAs per sequence and
+// value head) walks the chunks in order: three products per chunk (U, O, the state update), the gated RMSNorm of O, and the output.  The products
 // are 64 x 128 x 128 at most and sit on a serial chain.  Written with the value index as the rows of every product (U^T, O^T, S), each
 // one's accumulator IS the next one's left operand, register for register, so a warp carries 16 values through all three without
 // meeting another warp or shared memory; only the right operands come from there (ldmatrix), the next chunk's copied while this one
 // is worked on.  Warp-level mma (bf16 in, fp32 out) rather than tcgen05: a TMEM round trip per link of the chain would cost more than
-// the tiles themselves.  3001 tokens, 32 heads: 929 us with every link staged through shared memory, 359 us in this form, bound by the
-// rate of the warp-level mma (1792 of them per chunk on one SM); the preparation 246 -> 184 us.
+// the tiles themselves.  3001 tokens, 32 heads: 929 us with every link staged through shared memory, 359 us in this form on one SM per
+// head, bound by the rate of the warp-level mma (1792 of them per chunk, two warps on each tensor core), 322 us with a head's values
+// over a cluster of two CTAs; the preparation 246 -> 150 us.
 //
 // The reference's counterpart is the chunked scan of cuda/llm/cuda_llm_runner.c:8128 (batch_deltanet_scan_f32) and its test
 // cuda/llm/scan/deltanet_chunk_test.c; the per-token recurrence is common/transformer.h:2829-2851.
@@ -107,28 +108,44 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
   const size_t ws = (size_t)cb * a.dt_rank + h;
 
   // rows of the chunk: L2-normalised q (scaled by 1 / sqrt(d)) and k, v transposed; tokens past the end are zero rows
-  for (int i = warp; i < kDnC; i += kDnThreads / 32) {
-    const int t = t0 + i;
-    float q4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f}, v4[4] = {0.f, 0.f, 0.f, 0.f};
-    if (t < t1) {
-      const __nv_bfloat16* row = a.qkv + (size_t)t * a.ld_qkv;
-      const uint2 qr = *reinterpret_cast<const uint2*>(row + q_off + 4 * lane);
-      const uint2 kr = *reinterpret_cast<const uint2*>(row + k_off + 4 * lane);
-      const uint2 vr = *reinterpret_cast<const uint2*>(row + v_off + 4 * lane);
-      const __nv_bfloat16* qb = reinterpret_cast<const __nv_bfloat16*>(&qr);
-      const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(&kr);
-      const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(&vr);
+  // (warp w: rows 8 w .. 8 w + 7, all requested before the first is used; v leaves as eight tokens of a channel at a time)
+  {
+    uint2 qr[8], kr[8], vr[8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { q4[e] = __bfloat162float(qb[e]); k4[e] = __bfloat162float(kb[e]); v4[e] = __bfloat162float(vb[e]); }
+    for (int r = 0; r < 8; ++r) {
+      const int t = t0 + 8 * warp + r;
+      qr[r] = kr[r] = vr[r] = make_uint2(0u, 0u);
+      if (t < t1) {
+        const __nv_bfloat16* row = a.qkv + (size_t)t * a.ld_qkv;
+        qr[r] = *reinterpret_cast<const uint2*>(row + q_off + 4 * lane);
+        kr[r] = *reinterpret_cast<const uint2*>(row + k_off + 4 * lane);
+        vr[r] = *reinterpret_cast<const uint2*>(row + v_off + 4 * lane);
+      }
     }
-    const float qs = dn_warp_sum(q4[0] * q4[0] + q4[1] * q4[1] + q4[2] * q4[2] + q4[3] * q4[3]);
-    const float ks = dn_warp_sum(k4[0] * k4[0] + k4[1] * k4[1] + k4[2] * k4[2] + k4[3] * k4[3]);
-    const float qsc = rsqrtf(qs + a.eps) * rsqrtf((float)kDnD), ksc = rsqrtf(ks + a.eps);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int i = 8 * warp + r;
+      const __nv_bfloat16* qb = reinterpret_cast<const __nv_bfloat16*>(&qr[r]);
+      const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(&kr[r]);
+      float q4[4], k4[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { q4[e] = __bfloat162float(qb[e]); k4[e] = __bfloat162float(kb[e]); }
+      const float qs = dn_warp_sum(q4[0] * q4[0] + q4[1] * q4[1] + q4[2] * q4[2] + q4[3] * q4[3]);
+      const float ks = dn_warp_sum(k4[0] * k4[0] + k4[1] * k4[1] + k4[2] * k4[2] + k4[3] * k4[3]);
+      const float qsc = rsqrtf(qs + a.eps) * rsqrtf((float)kDnD), ksc = rsqrtf(ks + a.eps);
+      *reinterpret_cast<uint2*>(sQ + i * kDnLd + 4 * lane) = make_uint2(pack_bf16x2(q4[0] * qsc, q4[1] * qsc), pack_bf16x2(q4[2] * qsc, q4[3] * qsc));
+      *reinterpret_cast<uint2*>(sK + i * kDnLd + 4 * lane) = make_uint2(pack_bf16x2(k4[0] * ksc, k4[1] * ksc), pack_bf16x2(k4[2] * ksc, k4[3] * ksc));
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      sQ[i * kDnLd + 4 * lane + e] = __float2bfloat16(q4[e] * qsc);
-      sK[i * kDnLd + 4 * lane + e] = __float2bfloat16(k4[e] * ksc);
-      sVT[(4 * lane + e) * kDnLc + i] = __float2bfloat16(v4[e]);
+      uint4 o;
+      uint32_t* po = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t lo = e < 2 ? vr[2 * u].x : vr[2 * u].y, hi = e < 2 ? vr[2 * u + 1].x : vr[2 * u + 1].y;
+        po[u] = __byte_perm(lo, hi, e & 1 ? 0x7632 : 0x5410);
+      }
+      *reinterpret_cast<uint4*>(sVT + (4 * lane + e) * kDnLc + 8 * warp) = o;
     }
   }
   if (tid < kDnC) {
@@ -146,7 +163,16 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
   __syncthreads();
   if (tid == 0) {
     float acc = 0.f;
-    for (int i = 0; i < kDnC; ++i) { acc += sc[i]; sc[i] = acc; }
+    for (int i0 = 0; i0 < kDnC; i0 += 16) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(sc + i0 + 4 * u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        v[u].x = acc += v[u].x; v[u].y = acc += v[u].y; v[u].z = acc += v[u].z; v[u].w = acc += v[u].w;
+        *reinterpret_cast<float4*>(sc + i0 + 4 * u) = v[u];
+      }
+    }
   }
   __syncthreads();
   const float c_last = sc[kDnC - 1];
@@ -298,10 +324,11 @@ dn_chunk_prep_kernel(const DnChunkArgs a) {
   if (tid == 0) a.glast[ws] = __expf(c_last);
 }
 
-// One stage of the scan's operands in shared memory (bf16): exp(c) Q and -(T diag(exp c) K) [token][key], decayed keys [key][token], T V [value][token], M
-constexpr int kScanNw = kDnC * kDnLd, kScanKd = 2 * kDnC * kDnLd, kScanUv = kScanKd + kDnD * kDnLc, kScanM = kScanUv + kDnD * kDnLc;
-constexpr int kScanStage = kScanM + kDnC * kDnLc;
-constexpr int kScanSmem = 2 * kScanStage * 2 + kDnC * kDnLf * 4;
+// One stage of the scan's operands in shared memory (bf16): exp(c) Q and -(T diag(exp c) K) [token][key], decayed keys [key][token], M, T V [value][token]
+constexpr int kScanNw = kDnC * kDnLd, kScanKd = 2 * kDnC * kDnLd, kScanM = kScanKd + kDnD * kDnLc, kScanUv = kScanM + kDnC * kDnLc;
+// NS CTAs share a head: each has 128 / NS values, and finishes (norm, gate) 64 / NS tokens of a chunk, in one or (NS > 1) two buffers of output rows.
+__host__ __device__ constexpr int scan_stage(int ns) { return kScanUv + kDnD / ns * kDnLc; }
+__host__ __device__ constexpr int scan_smem(int ns) { return 2 * scan_stage(ns) * 2 + (ns > 1 ? 2 : 1) * kDnC / ns * kDnLf * 4; }
 
 __device__ __forceinline__ void dn_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -340,15 +367,18 @@ __device__ __forceinline__ void dn_product(float (*c)[4], const uint32_t (*a)[4]
   }
 }
 
-__global__ void __launch_bounds__(kDnThreads, 1)
+template <int NS>
+__global__ void __launch_bounds__(kDnThreads / NS, 1)
 dn_chunk_scan_kernel(const DnChunkArgs a) {
+  constexpr int THREADS = kDnThreads / NS, STAGE = scan_stage(NS), TOK = kDnC / NS;
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(128) uint8_t dn_smem[];
-  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(dn_smem);        // [2][kScanStage]
-  float* sO = reinterpret_cast<float*>(ring + 2 * kScanStage);             // [64 tokens][kDnLf]
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(dn_smem);        // [2][STAGE]
+  float* sO = reinterpret_cast<float*>(ring + 2 * STAGE);                  // [1 or 2][TOK tokens][kDnLf]
 
-  const int h = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x / NS, rank = blockIdx.x % NS, s = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int lwarp = tid >> 5, warp = rank * (THREADS / 32) + lwarp;        // warp of the head: values 16 warp .., tokens 8 warp .. of a chunk
   const int seq_t0 = a.cu_q[s], seq_t1 = a.cu_q[s + 1];
   if (seq_t1 <= seq_t0) return;
   int cb = 0;
@@ -357,21 +387,21 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
 
   auto fetch = [&](int ci) {                                               // chunk ci -> its stage, 16 bytes per copy
     const size_t ws = (size_t)(cb + ci) * a.dt_rank + h;
-    __nv_bfloat16* st = ring + (ci & 1) * kScanStage;
+    __nv_bfloat16* st = ring + (ci & 1) * STAGE;
     const __nv_bfloat16* gq = a.gq + ws * kDnC * kDnD;
     const __nv_bfloat16* nw = a.nw + ws * kDnC * kDnD;
     const __nv_bfloat16* kd = a.kdt + ws * kDnC * kDnD;
-    const __nv_bfloat16* uv = a.uv + ws * kDnC * kDnD;
+    const __nv_bfloat16* uv = a.uv + ws * kDnC * kDnD + rank * (kDnD / NS) * kDnC;
     const __nv_bfloat16* mq = a.mqk + ws * kDnC * kDnC;
 #pragma unroll
-    for (int i = 0; i < kDnC * kDnD / 8 / kDnThreads; ++i) {
-      const int idx = tid + i * kDnThreads;
+    for (int i = 0; i < kDnC * kDnD / 8 / THREADS; ++i) {
+      const int idx = tid + i * THREADS;
       const int r = idx / (kDnD / 8) * kDnLd + 8 * (idx % (kDnD / 8)), q = idx / (kDnC / 8) * kDnLc + 8 * (idx % (kDnC / 8));
       dn_copy16(st + r, gq + 8 * idx);
       dn_copy16(st + kScanNw + r, nw + 8 * idx);
       dn_copy16(st + kScanKd + q, kd + 8 * idx);
-      dn_copy16(st + kScanUv + q, uv + 8 * idx);
-      if (i < kDnC * kDnC / 8 / kDnThreads) dn_copy16(st + kScanM + q, mq + 8 * idx);
+      if (i < kDnC * kDnD / NS / 8 / THREADS) dn_copy16(st + kScanUv + q, uv + 8 * idx);
+      if (i < kDnC * kDnC / 8 / THREADS) dn_copy16(st + kScanM + q, mq + 8 * idx);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -391,14 +421,19 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
   const uint32_t off_d = (uint32_t)(lrow * kDnLd + lk) * 2, off_c = (uint32_t)(lrow * kDnLc + lk) * 2;
   const float4 nwt = *reinterpret_cast<const float4*>(a.norm_w + 4 * lane);
 
+  if constexpr (NS > 1) {     // the other CTA runs: its shared memory may be written to
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
   for (int ci = 0; ci < n_chunks; ++ci) {
     const int t0 = seq_t0 + ci * kDnC, t1 = min(t0 + kDnC, seq_t1);
     const float g_last = a.glast[(size_t)(cb + ci) * a.dt_rank + h];
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();          // this chunk's tiles have landed; everyone is done with the other stage and with sO
     if (ci + 1 < n_chunks) fetch(ci + 1);
-    const __nv_bfloat16* stg = ring + (ci & 1) * kScanStage;
-    const uint32_t su = ring_u + (uint32_t)(ci & 1) * (kScanStage * 2);
+    const __nv_bfloat16* stg = ring + (ci & 1) * STAGE;
+    const uint32_t su = ring_u + (uint32_t)(ci & 1) * (STAGE * 2);
+    float* out_rows = sO + (NS > 1 ? (ci & 1) * TOK * kDnLf : 0);
 
     uint32_t aS[8][4];                                                     // the state in front of the chunk as a bf16 operand
 #pragma unroll
@@ -410,7 +445,7 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
       float U[8][4];
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
-        const __nv_bfloat16* p = stg + kScanUv + (16 * warp + g) * kDnLc + 8 * n + 2 * q;
+        const __nv_bfloat16* p = stg + kScanUv + (16 * lwarp + g) * kDnLc + 8 * n + 2 * q;
         const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + 8 * kDnLc));
         U[n][0] = lo.x; U[n][1] = lo.y; U[n][2] = hi.x; U[n][3] = hi.y;
       }
@@ -436,11 +471,19 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
           dn_mma(O[2 * p], aU[k], b[0], b[1]);
           dn_mma(O[2 * p + 1], aU[k], b[2], b[3]);
         }
-      float* o = sO + 2 * q * kDnLf + 16 * warp + g;
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
-        o[8 * n * kDnLf] = O[n][0]; o[(8 * n + 1) * kDnLf] = O[n][1];
-        o[8 * n * kDnLf + 8] = O[n][2]; o[(8 * n + 1) * kDnLf + 8] = O[n][3];
+        const int t = 8 * n + 2 * q;                                       // tokens t and t + 1 go to the CTA that finishes them
+        float* o = out_rows + (t % TOK) * kDnLf + 16 * warp + g;
+        if constexpr (NS == 1) {
+          o[0] = O[n][0]; o[kDnLf] = O[n][1]; o[8] = O[n][2]; o[kDnLf + 8] = O[n][3];
+        } else {
+          uint32_t r;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(o)), "r"(8 * n / TOK));
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(r + (uint32_t)((e & 1) * kDnLf + (e >> 1) * 8) * 4), "f"(O[n][e]) : "memory");
+        }
       }
     }
     uint2 zr[8];                                                           // gates of the tokens this warp will finish
@@ -449,7 +492,12 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
       const int t = t0 + 8 * warp + i;
       zr[i] = t < t1 ? *reinterpret_cast<const uint2*>(a.z + (size_t)t * a.ld_z + h * kDnD + 4 * lane) : make_uint2(0u, 0u);
     }
-    __syncthreads();          // the output rows are complete
+    // the output rows are complete.  (NS > 1: a CTA writes this buffer again two chunks on, behind a barrier at which the others arrive with this one read)
+    if constexpr (NS == 1) __syncthreads();
+    else {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
 
     // S = exp(c_last) S + U^T diag(exp(c_last - c_j)) K
 #pragma unroll
@@ -464,7 +512,7 @@ dn_chunk_scan_kernel(const DnChunkArgs a) {
     for (int i = 0; i < 8; ++i) {
       const int t = t0 + 8 * warp + i;
       if (t >= t1) break;
-      const float4 o = *reinterpret_cast<const float4*>(sO + (8 * warp + i) * kDnLf + 4 * lane);
+      const float4 o = *reinterpret_cast<const float4*>(out_rows + (8 * lwarp + i) * kDnLf + 4 * lane);
       const float ss = dn_warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w);
       const float sc = rsqrtf(ss / (float)kDnD + a.eps);
       const __nv_bfloat16* zb = reinterpret_cast<const __nv_bfloat16*>(&zr[i]);
@@ -527,12 +575,17 @@ GB_API int gb_deltanet_chunked(const void* qkv, int ld_qkv, const void* z, int l
   static bool attr_set = false;
   if (!attr_set) {
     GB_CUDA_OK(cudaFuncSetAttribute(dn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem));
-    GB_CUDA_OK(cudaFuncSetAttribute(dn_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem));
+    GB_CUDA_OK(cudaFuncSetAttribute(dn_chunk_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem(1)));
+    GB_CUDA_OK(cudaFuncSetAttribute(dn_chunk_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem(2)));
     attr_set = true;
   }
   launch_k(dn_chunk_prep_kernel, dim3((unsigned)chunks, dt_rank), kDnThreads, kPrepSmem, stream, g);
   GB_CUDA_OK(cudaGetLastError());
-  launch_k(dn_chunk_scan_kernel, dim3(dt_rank, n_seqs), kDnThreads, kScanSmem, stream, g);
+  // two CTAs per head where they all fit the GPU at once; else a second round would cost more than the shared tensor cores
+  if (2L * dt_rank * n_seqs <= sm_count())
+    GB_CUDA_OK(launch_k_cluster(dn_chunk_scan_kernel<2>, dim3(2 * dt_rank, n_seqs), dim3(kDnThreads / 2), (size_t)scan_smem(2), stream, 2u, g));
+  else
+    launch_k(dn_chunk_scan_kernel<1>, dim3(dt_rank, n_seqs), kDnThreads, scan_smem(1), stream, g);
   GB_CUDA_OK(cudaGetLastError());
   return 0;
 }

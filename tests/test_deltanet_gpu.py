@@ -109,6 +109,27 @@ def test_deltanet_chunked_scan(lens):
         assert _rel(got[cu[i]:cu[i + 1]], ref[cu[i]:cu[i + 1]]) < 2e-2, (i, lens[i])
 
 
+def test_deltanet_scan_with_one_and_two_ctas_per_head():
+    """A launch whose heads fill the GPU scans with a CTA per head, a small one with two: the same numbers, bit for bit."""
+    torch.manual_seed(6)
+    ds, ng, hv, n = 128, 2, 4, 24                     # 192 CTAs in pairs: more than SMs
+    lens = [48 + 7 * i for i in range(n)]
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    t = cu[-1]
+    qkv, z, ab = torch.randn(t, (2 * ng + hv) * ds, device="cuda").bfloat16(), torch.randn(t, hv * ds, device="cuda").bfloat16(), torch.randn(t, 2 * hv, device="cuda")
+    a, bias, nw = -(torch.rand(hv, device="cuda") * 2 + 0.1), torch.randn(hv, device="cuda") * 0.5, torch.rand(ds, device="cuda") + 0.5
+    st = torch.randn(n, hv, ds, ds, device="cuda") * 0.1
+    st1 = st.clone()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    got = dn.deltanet(qkv, z, ab, a, bias, nw, st, i32(cu), i32(list(range(n))), ng, hv, ds, 1e-6)
+    for i in range(n):
+        sl = slice(cu[i], cu[i + 1])
+        one = dn.deltanet(qkv[sl], z[sl], ab[sl], a, bias, nw, st1, i32([0, lens[i]]), i32([i]), ng, hv, ds, 1e-6)
+        assert torch.equal(one, got[sl]), i
+    _native.assert_status_ok()
+    assert torch.equal(st, st1)
+
+
 def test_sigmoid_gate_mul():
     torch.manual_seed(3)
     x = torch.randn(19, 512).bfloat16()
