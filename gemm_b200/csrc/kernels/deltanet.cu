@@ -38,7 +38,9 @@ ssm_conv_silu_kernel(const __nv_bfloat16* __restrict__ x, int ld_x, const float*
   constexpr int MK = K ? K : kMaxConvK;
   const int nh = K ? K - 1 : conv_k - 1;
   const int c = (blockIdx.y * 256 + threadIdx.x) * VEC;
-  float wk[MK][VEC];                                    // weights: no kernel of a step writes them
+  pdl_wait();
+  pdl_trigger();
+  float wk[MK][VEC];
 #pragma unroll
   for (int u = 0; u < VEC; ++u) {
     if constexpr (K == 4 && VEC == 4) {
@@ -49,8 +51,6 @@ ssm_conv_silu_kernel(const __nv_bfloat16* __restrict__ x, int ld_x, const float*
       for (int f = 0; f < MK; ++f) wk[f][u] = (f <= nh && c < channels) ? w[(size_t)(c + u) * (nh + 1) + f] : 0.f;
     }
   }
-  pdl_wait();
-  pdl_trigger();
   // tile -> sequence: running sum of the sequences' tile counts, 32 sequences at a time
   const int lane = threadIdx.x & 31;
   int tile = blockIdx.x, seq = -1, s_t0 = 0, s_t1 = 0;

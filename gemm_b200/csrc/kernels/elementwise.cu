@@ -57,8 +57,8 @@ struct RmsBcast {
 
 // One CTA per row.  Optional: residual[row] += delta[row] first (the sum is written back and is the
 // normalised input); optional MXFP8 output (e4m3 bytes + scale atoms) beside / instead of bf16.
-// A decode step's row is bound by latency: the weights are requested before the dependency wait (no kernel of a step writes them), and the K-split partial
-// sums or the experts' rows of all the thread's vectors in groups of independent loads, added in their order.  Against one load after another: a row of 5120
+// A decode step's row is bound by latency: the weights are requested with the row, and the K-split partial sums or the experts' rows of all the thread's
+// vectors in groups of independent loads, added in their order.  Against one load after another: a row of 5120
 // behind seven partials 7.2 -> 3.8 us, 32 rows of 4096 behind four 4.8 -> 2.9 us; 16384 rows of 2048 behind their experts' rows 180 -> 133 us, behind one
 // row each 66 -> 51 us (5.3 TB/s).
 // VPT: 8-element vectors per thread (hidden <= 256 * 8 * VPT).  SRC, what joins the residual: 0 = nothing or bf16 rows, 1 = partial sums, 2 = the experts' rows (an
@@ -71,14 +71,14 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __rest
                const float* __restrict__ partials, int n_partials, long partial_stride, const uint32_t* wait_flags, int wait_n,
                const uint32_t* epoch_ptr, KernelStatus* st, const __nv_bfloat16* __restrict__ comb_y, const int* __restrict__ comb_rows,
                const float* __restrict__ comb_w, int comb_k, int comb_ld, int part_inner, long part_inner_stride, const RmsBcast bc) {
+  pdl_wait();
+  pdl_trigger();
   const int row = blockIdx.x;
   const int nvec = hidden >> 3;
   bf16x8 wv[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i)
     if (threadIdx.x + i * 256 < nvec) wv[i] = *reinterpret_cast<const bf16x8*>(weight + (threadIdx.x + i * 256) * 8);
-  pdl_wait();
-  pdl_trigger();
   __shared__ int c_rows[16];
   __shared__ float c_w[16];
   if (SRC == 2) {

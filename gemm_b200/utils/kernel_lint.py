@@ -13,7 +13,9 @@ Rules (each has cost a GPU somewhere before it became a rule):
 * ``no-cluster-broadcast-load``  no TMA or bulk load that delivers its tile to several CTAs of a cluster at once (the PTX qualifier
   made of the words "multicast" and "cluster") in a file that runs on more than one GPU; files named in ``.gpurunignore.multi`` are
   exempt: they never travel to a multi-GPU run.  ``tcgen05.commit`` with that qualifier is not a load and is fine;
-* ``arch``           no ``wgmma`` (Hopper only; does not assemble for sm_100a).
+* ``arch``           no ``wgmma`` (Hopper only; does not assemble for sm_100a);
+* ``wait-first``     a kernel with a dependency wait (``pdl_wait``) reads no global memory in front of it: the kernel before it on the stream lets its
+  successor start before its own stores.  ``EARLY_WEIGHTS`` names the kernels that request weights there all the same, and why they may.
 
 The reference validates generated PTX strings without a GPU (cuda/ptx_validate.h: directives, braces, known mnemonics); here
 nvcc already rejects malformed inline PTX at build time, so the linter checks what the assembler cannot know.
@@ -35,6 +37,12 @@ INVENTORY = [("tcgen05.mma", r"tcgen05\.mma"), ("tcgen05.ld/st/cp", r"tcgen05\.(
              ("cp.async.bulk.tensor", r"cp\.async\.bulk\.tensor"), ("cp.async.bulk", r"cp\.async\.bulk(?!\.tensor)"),
              ("mbarrier", r"mbarrier\."), ("griddepcontrol", r"griddepcontrol\."), ("mma.sync / wmma", r"mma\.sync|wmma::"),
              ("peer / multimem", r"multimem\.|peer_")]
+
+
+# Kernels that request weights in front of their dependency wait.  Their entry points say that these weights must not come from the launch directly
+# before (gemm_tc_kernel: or that the launch says so).
+EARLY_WEIGHTS = {"gemm_tc_kernel", "qgemv_kernel", "moe_prep_kernel"}
+GLOBAL_LOADS = r"\b(?:tma_load\w*|bulk_load\w*|load8|ld_\w+|__ldg|__ldcg|stage_slice)\s*[(<]"
 
 
 def strip_comments(text: str) -> str:
@@ -99,15 +107,44 @@ def loops(text: str):
         yield text.count("\n", 0, m.start()) + 1, header, body
 
 
-def kernels(text: str):
-    """(name, body) of every __global__ function."""
-    for m in re.finditer(r"__global__[^;{]*?\b(\w+)\s*\(", text):
-        p1 = _match_paren(text, m.end() - 1)
+def kernel_parts(text: str):
+    """(name, parameters, body) of every __global__ function."""
+    for m in re.finditer(r"__global__[^;{(]*?\b(\w+)\s*\(", text):
+        name, p0 = m.group(1), m.end() - 1
+        if name == "__launch_bounds__":                  # the function's own name follows the bounds
+            n = re.compile(r"[^;{(]*?\b(\w+)\s*\(").match(text, _match_paren(text, p0) + 1)
+            if n is None:
+                continue
+            name, p0 = n.group(1), n.end() - 1
+        p1 = _match_paren(text, p0)
         j = text.find("{", p1)
         semi = text.find(";", p1)
         if j < 0 or (0 <= semi < j):
             continue
-        yield m.group(1), text[j: _match_brace(text, j) + 1]
+        yield name, text[p0 + 1: p1], text[j: _match_brace(text, j) + 1]
+
+
+def kernels(text: str):
+    """(name, body) of every __global__ function."""
+    for name, _, body in kernel_parts(text):
+        yield name, body
+
+
+def reads_before_wait(params: str, body: str) -> List[str]:
+    """Pieces of ``body`` in front of its ``pdl_wait`` that read global memory: load helpers, and pointer parameters or pointer fields of a parameter
+    that are subscripted or dereferenced."""
+    at = re.search(r"\bpdl_wait\s*\(", body)
+    if at is None:
+        return []
+    pats = [GLOBAL_LOADS]
+    for p in params.split(","):
+        n = re.search(r"(\w+)\s*(?:\[[^\]]*\])?\s*$", p)
+        if n is None:
+            continue
+        ptr = "*" in p
+        name = re.escape(n.group(1)) + ("" if ptr else r"\.\w+")
+        pats += [r"\b%s\s*\[" % name, r"\*\s*reinterpret_cast<[^>]*>\(\s*%s\b" % name] + ([r"\*\s*%s\b" % name] if ptr else [])
+    return [m.group(0) for pat in pats for m in re.finditer(pat, body[: at.start()])]
 
 
 def helper_map(header_text: str) -> Dict[str, str]:
@@ -139,6 +176,10 @@ def lint_text(name: str, raw: str, multi_gpu: bool = True, helpers: Dict[str, st
     for kname, body in kernels(text):
         if re.search(r"\btmem_alloc\s*\(", body) and not re.search(r"\btmem_dealloc\s*\(", body):
             out.append({"rule": "tmem-paired", "file": name, "line": 0, "what": f"kernel {kname} allocates tensor memory and never frees it"})
+    for kname, params, body in kernel_parts(text):
+        if kname not in EARLY_WEIGHTS:
+            for what in reads_before_wait(params, body):
+                out.append({"rule": "wait-first", "file": name, "line": 0, "what": f"kernel {kname} reads global memory before pdl_wait: {what}"})
     if "tcgen05.alloc" in text and not ("tcgen05.dealloc" in text and "tcgen05.relinquish_alloc_permit" in text):
         out.append({"rule": "tmem-paired", "file": name, "line": 0, "what": "tcgen05.alloc without dealloc / relinquish_alloc_permit"})
     if multi_gpu:

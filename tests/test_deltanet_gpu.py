@@ -5,6 +5,7 @@ import torch
 from gemm_b200 import _native
 from gemm_b200.ops import deltanet as dn
 from gemm_b200.ops import elementwise as ew
+from gemm_b200.ops import gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -47,6 +48,22 @@ def test_conv_silu_tiles(ch, ck, wide, off):
     assert (got.float().cpu() - ref.float()).abs().max() <= 2 ** -7 * ref.float().abs().max()
     assert _rel(got, ref) < 2 ** -9
     assert torch.equal(st_gpu.cpu(), st)
+
+
+def test_conv_silu_taps_of_the_launch_before():
+    """The taps may be the result of the kernel launched just before, which lets its successor start before it stores."""
+    torch.manual_seed(7)
+    ch, ck, k = 12288, 4, 512
+    a, b = torch.randn(ch, k, device="cuda").bfloat16(), (torch.randn(ck, k, device="cuda") * k ** -0.5).bfloat16()
+    x, st = torch.randn(8, ch, device="cuda").bfloat16(), torch.randn(1, ck - 1, ch, device="cuda")
+    cu, slots = torch.tensor([0, 8], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    w = gemm.linear(a, b, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    want = dn.conv_silu(x, w.clone(), st.clone(), cu, slots)
+    s2 = st.clone()
+    torch.full((ch, ck), float("nan"), device="cuda")                                        # what the allocator hands out next
+    torch.cuda.synchronize()
+    assert torch.equal(dn.conv_silu(x, gemm.linear(a, b, out_dtype=torch.float32), s2, cu, slots), want)
 
 
 @pytest.mark.parametrize("ds,ng,hv", [(64, 2, 4), (128, 2, 6)])

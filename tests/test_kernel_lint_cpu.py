@@ -35,3 +35,16 @@ def test_rules_fire():
     assert _rules(commit) == []
     assert _rules('void f() { asm volatile("wgmma.mma_async.sync.aligned.m64n128k16.f32.bf16.bf16 ..."); }') == ["arch"]
     assert _rules("// while (ld_acquire_gpu(f) == 0) {}\n/* tmem_alloc( */ void f() {}") == []
+
+
+def test_reads_in_front_of_the_dependency_wait():
+    # weights may come out of the kernel launched just before, which lets its successor start before it stores
+    head = "template <int N>\n__global__ void __launch_bounds__(256)\nk(const float* __restrict__ w, const Args a, float* out) "
+    assert _rules(head + "{ const float x = w[threadIdx.x]; pdl_wait(); pdl_trigger(); out[0] = x; }") == ["wait-first"]
+    assert _rules(head + "{ const float4 x = *reinterpret_cast<const float4*>(w + 4); pdl_wait(); }") == ["wait-first"]
+    assert _rules(head + "{ const float x = a.tab[3]; pdl_wait(); }") == ["wait-first"]
+    assert _rules(head + "{ bulk_load(smem, a.w, 16, bar); pdl_wait(); }") == ["wait-first"]
+    assert _rules(head + "{ float t[4]; const int n = 2 * a.rows; pdl_wait(); t[0] = w[n]; out[0] = a.tab[1] + *w; }") == []
+    assert _rules(head + "{ out[0] = w[0]; }") == []                   # without a wait: launched in plain stream order
+    named = [n for n, _, _ in kl.kernel_parts(kl.strip_comments(head + "{ }"))]
+    assert named == ["k"]

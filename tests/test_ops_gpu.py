@@ -4,7 +4,7 @@ import torch
 
 from gemm_b200 import _native
 from gemm_b200.ops import elementwise as ew
-from gemm_b200.ops import moe, mxfp8, sampling
+from gemm_b200.ops import moe, mxfp8, quant, sampling
 
 pytestmark = pytest.mark.gpu
 
@@ -26,6 +26,22 @@ def test_rmsnorm(rows, hidden):
     w = (1 + 0.1 * torch.randn(hidden, device="cuda")).bfloat16()
     y = ew.rmsnorm(x, w, 1e-6)
     assert _rel(y, ew.rmsnorm_ref(x, w, 1e-6)) < 4e-3
+
+
+@pytest.mark.parametrize("hidden", [1024, 8192])
+def test_rmsnorm_weight_of_the_launch_before(hidden):
+    """The weight may be the result of the kernel launched just before, which lets its successor start before it stores."""
+    torch.manual_seed(2)
+    n = 4096
+    raw = quant.QuantWeight.from_float(torch.randn(n, hidden), "Q8_0", device="cuda")
+    x = torch.randn(64, hidden, device="cuda").bfloat16()
+    w = raw.dequantize()
+    torch.cuda.synchronize()
+    for row in (0, n // 2, n - 1):
+        want = ew.rmsnorm(x, w[row].clone(), 1e-6)
+        torch.full((n, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")          # what the allocator hands out next
+        torch.cuda.synchronize()
+        assert torch.equal(ew.rmsnorm(x, raw.dequantize()[row], 1e-6), want)
 
 
 def test_rmsnorm_residual_quant():
