@@ -811,13 +811,15 @@ struct GemmExtras {
 };
 
 // Flags of gb_gemm.
-enum { GEMM_MX = 1, GEMM_DUAL = 2, GEMM_QUANT_OUT = 4, GEMM_OUT_F32 = 8, GEMM_W_TILED = 16, GEMM_DUAL_RAW = 32, GEMM_GELU = 64, GEMM_CAPPED = 128, GEMM_GELU_ERF = 256 };
+enum { GEMM_MX = 1, GEMM_DUAL = 2, GEMM_QUANT_OUT = 4, GEMM_OUT_F32 = 8, GEMM_W_TILED = 16, GEMM_DUAL_RAW = 32, GEMM_GELU = 64, GEMM_CAPPED = 128, GEMM_GELU_ERF = 256, GEMM_W_FRESH = 512 };
 
 // Linear layer on tensor cores.
 //   w        [w_rows, k] row-major (bf16, or e4m3 bytes when GEMM_MX), w_rows = groups * w_rows_per_group
 //   x        [x_rows, k] row-major, same element type as w
 //   out      [*, ldo]    bf16 (default), f32 (GEMM_OUT_F32) or e4m3 + out_sf (GEMM_QUANT_OUT)
 //   tn       token tile: 16, 32, 64, 128 or 256 (256: non-DUAL without quantised output only)
+// GEMM_W_FRESH: w or sfa is written by the launch directly before this one (otherwise a launch with token tiles of at most 64 reads them while that one may
+// still run).
 // Grouped mode (num_groups > 0): seg_start / seg_count are device arrays; seg_start[g] must be a
 // multiple of min(tn, 128); `max_rows` bounds the segment buffer (TMA extent).
 GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, int m_tok, int ldw, int ldx, int ldo,
@@ -863,7 +865,7 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
   {
     static int early = -1;                      // GB_GEMM_EARLY_WEIGHTS=0 switches the early weight requests off (A/B measurements)
     if (early < 0) { const char* e = getenv("GB_GEMM_EARLY_WEIGHTS"); early = (e != nullptr && atoi(e) == 0) ? 0 : 1; }
-    a.early_weights = early;
+    a.early_weights = early && !(flags & GEMM_W_FRESH);
   }
   a.dual_raw = (flags & GEMM_DUAL_RAW) ? 1 : 0;
   const bool gelu = flags & GEMM_GELU;

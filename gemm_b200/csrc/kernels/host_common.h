@@ -48,8 +48,8 @@ int sm_count();   // SMs of the current device (cached per device)
 
 // Programmatic dependent launch: when on (default; gb_set_pdl(0) or GB_PDL=0 turns it off), every kernel of this library
 // is launched with the "programmatic stream serialization" attribute.  Each kernel signals
-// griddepcontrol.launch_dependents as soon as it starts and executes griddepcontrol.wait before its first access to
-// global memory, so the launch latency and the prologue (barrier init, TMEM allocation, descriptor prefetch) of kernel
+// griddepcontrol.launch_dependents as soon as its own griddepcontrol.wait has returned, and executes that wait before its first access to
+// global memory (three kernels request resident weights earlier, see pdl_wait), so the launch latency and the prologue (barrier init, TMEM allocation, descriptor prefetch) of kernel
 // N+1 overlap the tail of kernel N while all memory dependencies stay those of a plain stream.
 bool pdl_enabled();
 

@@ -50,6 +50,8 @@ __device__ __forceinline__ void report_status(KernelStatus* st, int code, int wh
 // Programmatic dependent launch.  pdl_trigger(): the next kernel of the stream may be scheduled (it still blocks in its
 // own pdl_wait() until this grid has completed and its writes are visible).  pdl_wait(): returns once every kernel this
 // one depends on has completed; nothing before it may touch global memory that an earlier kernel writes or reads.
+// (gemm_tc_kernel, qgemv_kernel and moe_prep_kernel request weights there: these must have been written before the launch directly in front of
+// theirs, or, gemm_tc_kernel, the launch says GEMM_W_FRESH.)
 // Both are no-ops for a kernel launched without the attribute.  Kernels here trigger right AFTER their own wait: a trigger
 // at kernel entry let whole chains of not-yet-runnable grids become resident at once and measured slower than plain
 // stream order on the decode step.

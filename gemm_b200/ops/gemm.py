@@ -17,7 +17,7 @@ from .. import _native
 from . import mxfp8
 from .mxfp8 import MxTensor
 
-GEMM_MX, GEMM_DUAL, GEMM_QUANT_OUT, GEMM_OUT_F32, GEMM_W_TILED, GEMM_DUAL_RAW, GEMM_GELU, GEMM_CAPPED, GEMM_GELU_ERF = 1, 2, 4, 8, 16, 32, 64, 128, 256
+GEMM_MX, GEMM_DUAL, GEMM_QUANT_OUT, GEMM_OUT_F32, GEMM_W_TILED, GEMM_DUAL_RAW, GEMM_GELU, GEMM_CAPPED, GEMM_GELU_ERF, GEMM_W_FRESH = 1, 2, 4, 8, 16, 32, 64, 128, 256, 512
 GATE_ACTS = ("silu", "gelu_tanh", "capped")         # activations of a gated feed-forward, by the code the kernels use
 GATE_ACT_CODE = {a: i for i, a in enumerate(GATE_ACTS)}
 
@@ -144,9 +144,11 @@ def _launch(w, x, out, n_out, k, m_tok, ldw, ldx, ldo, flags, tn, num_groups=0, 
 # --------------------------------------------------------------------------------------------- bf16
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
            out_dtype=torch.bfloat16, tn: Optional[int] = None, split_k: bool = False, w_tiled: bool = False,
-           silu_rows: int = 0, gelu: bool = False) -> torch.Tensor:
+           silu_rows: int = 0, gelu: bool = False, w_fresh: bool = False) -> torch.Tensor:
     """``x [M, K] @ w[N, K]^T`` (bf16 operands, fp32 accumulate).  ``w_tiled``: ``w`` is in ``mxfp8.tile_weight`` layout.  ``silu_rows``: SiLU on
-    that many leading output features, in the epilogue; ``gelu``: the exact GELU on all of them (bf16 results)."""
+    that many leading output features, in the epilogue; ``gelu``: the exact GELU on all of them (bf16 results).  ``w_fresh``: ``w`` is the result of the
+    kernel launched directly before this one.  Launches of up to 64 tokens, here and in the functions below, otherwise request weights while that
+    kernel still runs."""
     m, k = x.shape
     n = w.shape[0]
     if not x.is_cuda:
@@ -159,7 +161,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=x.device)
-    flags = (GEMM_OUT_F32 if out.dtype == torch.float32 else 0) | (GEMM_W_TILED if w_tiled else 0) | (GEMM_GELU_ERF if gelu else 0)
+    flags = (GEMM_OUT_F32 if out.dtype == torch.float32 else 0) | (GEMM_W_TILED if w_tiled else 0) | (GEMM_GELU_ERF if gelu else 0) | (GEMM_W_FRESH if w_fresh else 0)
     tn = tn or (max(128, pick_tn(m)) if silu_rows else pick_tn(m))
     ex = _splitk_extras(n, m, k, tn, False, x.device, split_k) if not (silu_rows or gelu) else GemmExtras()
     if silu_rows:

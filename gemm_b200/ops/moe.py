@@ -156,7 +156,8 @@ def prep_hidden(h: torch.Tensor, w: torch.Tensor, k: int, n_exp: int, align: int
     Returns ``(ids, weights, MoePlan, rows)``; ``rows`` is an ``MxTensor`` (MXFP8 with scale atoms in the ``align``-row layout,
     ``align`` 32 or 128) when ``quantize`` else a bf16 tensor ``[capacity, hidden]``.  Rows of the buffer that no (token, expert)
     pair maps to are left unwritten: the grouped GEMM computes them and drops them.  ``n_exp`` is the number of experts the plan
-    covers (the local count with ``local_range``).  ``wait_*``: flags of peer GPUs to wait for before the tokens are read."""
+    covers (the local count with ``local_range``).  ``wait_*``: flags of peer GPUs to wait for before the tokens are read.  ``w`` is read
+    while the launch in front of this one may still run: it must not be that launch's result."""
     from . import elementwise as ew
     from .mxfp8 import MxTensor
     t, hid = h.shape

@@ -32,7 +32,8 @@ GEMV_MAX_TOKENS = 4
 @dataclass
 class QTensor:
     """A ``[rows, k]`` matrix as tiled ggml blocks: ``data`` uint8 ``[ceil(rows / 128), k / 256, tile_bytes]``; rows past ``rows``
-    (padding up to the tile) are zero blocks."""
+    (padding up to the tile) are zero blocks.  The GEMV requests them while the launch in front of it may still run: they must not be
+    that launch's result."""
     data: torch.Tensor
     ggml_type: int
     rows: int

@@ -72,4 +72,4 @@ def linear_quant(x: torch.Tensor, w: QuantWeight, out_dtype=torch.bfloat16) -> t
         _native.check(rc, "gb_gemv_quant")
         return y if out_dtype == torch.float32 else y.to(out_dtype)
     from . import gemm
-    return gemm.linear(x, w.dequantize(), out_dtype=out_dtype)
+    return gemm.linear(x, w.dequantize(), out_dtype=out_dtype, w_fresh=True)

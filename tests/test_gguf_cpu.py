@@ -117,3 +117,17 @@ def test_gguf_rejects_garbage(tmp_path):
     p.write_bytes(b"NOPE" + b"\x00" * 64)
     with pytest.raises(IOError):
         gguf.GGUFFile(str(p))
+
+
+def test_weights_dequantised_in_front_of_a_product_are_waited_for(monkeypatch):
+    """``linear_quant`` above eight rows: the dequantised weights come from the launch directly before, so the product may not request them early."""
+    from gemm_b200.ops import gemm, quant
+
+    class Rows:
+        shape, is_cuda = (20, 256), True
+
+    seen = {}
+    monkeypatch.setattr(quant.QuantWeight, "dequantize", lambda self: "dequantised")
+    monkeypatch.setattr(gemm, "linear", lambda x, w, **kw: seen.update(kw, w=w))
+    quant.linear_quant(Rows(), quant.QuantWeight(None, 8, 64, 256))
+    assert seen["w"] == "dequantised" and seen["w_fresh"] is True

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from gemm_b200.ops import quant
+from gemm_b200.ops import gemm, quant
 from gemm_b200.utils import gguf
 
 pytestmark = pytest.mark.gpu
@@ -58,3 +58,19 @@ def test_linear_quant(t, m):
     ref = x.float() @ wf.t()
     tol = 2e-3 if m <= 8 else 1.5e-2          # the large-batch path rounds the weights to bf16 first
     assert ((y - ref).norm() / (ref.norm() + 1e-9)).item() < tol
+
+
+@pytest.mark.parametrize("m", [9, 33, 64])
+def test_linear_quant_waits_for_its_weights(m):
+    """The product's launch directly follows the one that dequantises its weights."""
+    torch.manual_seed(1)
+    rows, k = 4096, 4096
+    w = quant.QuantWeight(_random_blocks("Q8_0", rows, k).cuda(), gguf.type_id("Q8_0"), rows, k)
+    x = (torch.randn(m, k, device="cuda") * 0.3).bfloat16()
+    wf = w.dequantize()
+    torch.cuda.synchronize()
+    want = gemm.linear(x, wf)
+    for _ in range(3):
+        torch.full((rows, k), float("nan"), dtype=torch.bfloat16, device="cuda")          # what the allocator hands out next
+        torch.cuda.synchronize()
+        assert torch.equal(quant.linear_quant(x, w), want)
