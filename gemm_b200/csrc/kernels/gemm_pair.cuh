@@ -5,7 +5,7 @@
 // a cluster work on a tile of 256 features and up to 256 tokens: each holds the weights of 128 features (gate and up rows: two MMAs) and HALF of the token rows,
 // and the pair's MMA reads both halves, so a token row is staged once for 256 features: 900 cycles of shared memory for 1024 of the tensor core.  The
 // accumulators fill TMEM; eight epilogue warps take everything out of it before they store, so that the next tile starts early.  12288 features, k = 4096:
-// 8300 tokens 1765 -> 1205 us (1386 TFLOP/s), 768 tokens 183 -> 115 us, 512 tokens 144 -> 105 us, 130 tokens 86 -> 66 us.
+// 8300 tokens 1765 -> 1205 us (1386 TFLOP/s), 3000 tokens 675 -> 492 us, 768 tokens 168 -> 120 us, 129 tokens 84 -> 64 us (pair_pays: where it is the faster form).
 // (Products with one accumulator stay on the kernel of gemm_tc.cu, whose 256-token tile is not bound by shared memory: 8300 tokens by 6144 features 311 us there,
 // 328 us in this form, which starts 4 us later, behind the cluster's barriers.)
 //
@@ -243,6 +243,24 @@ inline int pair_tile_tokens(int m_tok, int n_blocks, int pairs) {
     if (best_cost < 0 || cost < best_cost) { best = tn; best_cost = cost; }
   }
   return best;
+}
+
+// Whether the pair form is the faster one of a gate / up projection (`n_out` features of `k`), against one SM per 128 features and 128 tokens.
+// Both forms timed in turn, in streams of launches that find their weights in memory: 512 to 25600 features, k 512 to 8192, 65 to 3000 tokens (us, one SM / pairs).
+//  * Up to 96 tokens: one SM (3072 x 1024, 65 tokens: 20.6 / 23.8; 12288 x 4096, 80 tokens: 54.9 / 58.9).
+//  * One round of tiles in either form: pairs, which end earlier, in the readout (3072 x 1024, 256 tokens: 23.6 / 21.3).  Not for long k, where their longer steps
+//    outweigh that (2048 x 8192, 384 tokens: 80.4 / 81.0), nor where single tiles fill the SMs (6144 x 2048, 320 tokens: 33.3 / 34.0) or up to 128 tokens stay one tile
+//    (10240 x 2560, 112 tokens: 41.1 / 45.1).
+//  * More rounds: a round of pairs costs 1.17 (160 tokens) to 1.30 (256) of a round of single tiles (12288 x 4096: 320 tokens, two rounds each, 90 / 101; 512 tokens,
+//    three and two, 127 / 104; 25600 x 5120, 256 tokens, three and two, 185 / 143).
+// Over those 502 sizes the choice takes 0.1 % longer than the better form of each, at worst 6 %.
+inline bool pair_pays(int n_out, int k, int m_tok, int sms) {
+  if (m_tok <= 96) return false;
+  const int pairs = sms / 2, n_blocks = n_out / 256, tn = pair_tile_tokens(m_tok, n_blocks, pairs);
+  const long single = 2l * n_blocks * ((m_tok + 127) / 128), single_rounds = (single + sms - 1) / sms;
+  const long rounds = ((long)n_blocks * ((m_tok + tn - 1) / tn) + pairs - 1) / pairs;
+  if (single_rounds == 1 && rounds == 1) return k <= 4096 && single <= 128 && (m_tok > 128 || tn <= 64);
+  return rounds * (95000 + 137 * tn) < 100000 * single_rounds;
 }
 
 // n_out a multiple of 256; tmW as gemm_tc.cu builds it, tmX with a box of 128 rows.

@@ -915,10 +915,10 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
   a.m_tok_hint = num_groups == 0 ? m_tok : (tn <= 32 ? tn : 1 << 20);
   if (num_groups == 0 && m_tok <= 0) return 0;
 
-  // SiLU gate / up projections of more than 64 tokens run on SM pairs (gemm_pair.cuh says why, and what both sides measure)
+  // SiLU gate / up projections of prefill-sized batches run on SM pairs where pair_pays says so (gemm_pair.cuh: why, and what both sides measure)
   if (dual && !mx && !qo && tn >= 128 && num_groups == 0 && n_out % 256 == 0 && up_row_offset % 128 == 0 && a.splits <= 1 && row_map == nullptr &&
       row_scale == nullptr && bias == nullptr && a.amax_val == nullptr && !a.out_f32 && !gelu && !capped && !a.dual_raw && a.wait_n == 0 &&
-      a.peer_region_rows == 0 && a.peer_bcast == 0 && a.signal_n == 0 && a.out_bytes != 0) {
+      a.peer_region_rows == 0 && a.peer_bcast == 0 && a.signal_n == 0 && a.out_bytes != 0 && pair_pays(n_out, k, m_tok, sm_count())) {
     CUtensorMap tmH;
     if (make_tmap_2d(&tmH, x, dt, (uint64_t)k, (uint64_t)x_rows, (uint64_t)ldx * esz, box_k, 128, TM_SW_128)) return -1;
     PairArgs pa;
@@ -980,3 +980,6 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
 #undef GB_DISPATCH
   return fail("gemm: unsupported variant%s (tn=%ld flags=%ld)", "", (long)tn, (long)flags);
 }
+
+// Whether a SiLU gate / up projection of these sizes takes the pair kernel on a GPU of `sms` SMs (n_out a multiple of 256).
+GB_API int gb_gemm_takes_pairs(int n_out, int k, int m_tok, int sms) { return pair_pays(n_out, k, m_tok, sms) ? 1 : 0; }

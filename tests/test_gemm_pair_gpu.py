@@ -10,6 +10,8 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [(65, 256, 64), (96, 256, 4096), (129, 512, 128), (257, 512, 72), (300, 768, 320), (511, 256, 1024), (2049, 1024, 520), (288, 4096, 4096), (5000, 1280, 256),
           (2600, 6144, 448)]
+# token counts that the pairs leave to a CTA per tile (and the first ones past them), features that are no whole number of pairs' blocks, two rounds in either form
+EDGES = [(80, 3072, 64), (96, 1024, 128), (97, 1024, 128), (128, 256, 192), (112, 9728, 64), (300, 384, 320), (320, 12288, 64), (300, 2048, 4160), (320, 6144, 64)]
 WIDE = [(256, 18944, 64), (300, 18951, 128), (2048, 19200, 192), (2305, 24576, 64), (4500, 18944, 72)]
 
 
@@ -27,7 +29,24 @@ def _close(got, ref):
     assert ((got.float() - ref).abs() <= bound).all(), (got.float() - ref).abs().max()
 
 
-@pytest.mark.parametrize("m,n,k", SHAPES)
+def _kernels(call):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES + EDGES)
+def test_swiglu_takes_the_kernel_of_the_rule(m, n, k):
+    x, w = _inputs(m, 2 * n, k)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    names = _kernels(lambda: gemm.linear_swiglu(x, w))
+    pairs = n % 256 == 0 and _native.cuda().gb_gemm_takes_pairs(n, k, m, sms) == 1
+    assert len([s for s in names if ("gemm_pair_kernel" if pairs else "gemm_tc_kernel") in s]) == 1, names
+    assert pairs or not any("gemm_pair_kernel" in s for s in names), names
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES + EDGES)
 def test_swiglu(m, n, k):
     x, w = _inputs(m, 2 * n, k)
     y = x.float() @ w.float().t()
