@@ -916,7 +916,7 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
   if (num_groups == 0 && m_tok <= 0) return 0;
 
   // SiLU gate / up projections of prefill-sized batches run on SM pairs where pair_pays says so (gemm_pair.cuh: why, and what both sides measure)
-  if (dual && !mx && !qo && tn >= 128 && num_groups == 0 && n_out % 256 == 0 && up_row_offset % 128 == 0 && a.splits <= 1 && row_map == nullptr &&
+  if (dual && !mx && !qo && tn == 128 && num_groups == 0 && n_out % 256 == 0 && up_row_offset % 128 == 0 && a.splits <= 1 && row_map == nullptr &&
       row_scale == nullptr && bias == nullptr && a.amax_val == nullptr && !a.out_f32 && !gelu && !capped && !a.dual_raw && a.wait_n == 0 &&
       a.peer_region_rows == 0 && a.peer_bcast == 0 && a.signal_n == 0 && a.out_bytes != 0 && pair_pays(n_out, k, m_tok, sm_count())) {
     CUtensorMap tmH;

@@ -71,3 +71,12 @@ def test_linear_with_many_features(m, n, k, tiled, dtype):
     gemm.linear(x, mxfp8.tile_weight(w) if tiled else w, bias=bias, out=out[:m], w_tiled=tiled)
     _close(out[:m], ref)
     assert (out[m] == 7).all()
+
+
+def test_gate_up_pairs_have_token_tiles_of_at_most_128():
+    x, w = _inputs(512, 6144, 256)
+    assert _native.cuda().gb_gemm_takes_pairs(3072, 256, 512, 148) == 1
+    with pytest.raises(RuntimeError, match="unsupported variant"):
+        gemm.linear_swiglu(x, w, tn=256)
+    with pytest.raises(RuntimeError, match="unsupported variant"):
+        gemm.linear_swiglu(x, w, tn=256, act="gelu_tanh")
