@@ -514,6 +514,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll 1
         for (int c = 0; c < TN; c += 16) {
           uint32_t r0[16];
+          __syncwarp();                            // rows past n_out left the round before early
           tmem_ld_x16(tacc + c, r0);
           tc_wait_ld();
           if (c >= t.valid || !n_ok) continue;
@@ -538,6 +539,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll 1
         for (int c = 0; c < TN; c += 16) {
           uint32_t r0[16], r1[16];
+          __syncwarp();
           tmem_ld_x16(tacc + c, r0);
           if (DUAL) tmem_ld_x16(tacc + TN + c, r1);
           tc_wait_ld();
@@ -638,6 +640,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll 1
         for (int c = 0; c < TN; c += 16) {
           uint32_t r0[16], r1[16];
+          __syncwarp();
           tmem_ld_x16(tacc + c, r0);
           if (DUAL) tmem_ld_x16(tacc + TN + c, r1);
           tc_wait_ld();
@@ -704,6 +707,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll 1
         for (int c = 0; c < TN; c += 16) {
           uint32_t r0[16], r1[16];
+          __syncwarp();
           tmem_ld_x16(tacc + c, r0);
           if (DUAL) tmem_ld_x16(tacc + TN + c, r1);
           tc_wait_ld();

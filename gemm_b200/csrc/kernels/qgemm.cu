@@ -210,6 +210,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const QGemmArgs args) {
 #pragma unroll 1
       for (int c = 0; c < TN; c += 16) {
         uint32_t r[16];
+        __syncwarp();                                      // rows past n_out left the round before early
         tmem_ld_x16(tacc + c, r);
         tc_wait_ld();
         if (c >= valid || !n_ok) continue;
@@ -440,6 +441,7 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
 #pragma unroll 1
       for (int c = 0; c < live; c += 16) {
         uint32_t r[16];
+        __syncwarp();                                      // rows past n_out left the round before early
         tmem_ld_x16(tacc + c, r);
         tc_wait_ld();
         if (!n_ok) continue;

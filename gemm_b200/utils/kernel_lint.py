@@ -14,6 +14,8 @@ Rules (each has cost a GPU somewhere before it became a rule):
   made of the words "multicast" and "cluster") in a file that runs on more than one GPU; files named in ``.gpurunignore.multi`` are
   exempt: they never travel to a multi-GPU run.  ``tcgen05.commit`` with that qualifier is not a load and is fine;
 * ``arch``           no ``wgmma`` (Hopper only; does not assemble for sm_100a);
+* ``converged``      an innermost loop that loads tensor memory (a warp-wide instruction, ``tmem_ld``) and goes round early by ``continue`` brings the warp
+  together (``__syncwarp``) in front of the load: lanes that left the last round early need not have met the others again;
 * ``wait-first``     a kernel with a dependency wait (``pdl_wait``) reads no global memory in front of it: the kernel before it on the stream lets its
   successor start before its own stores.  ``EARLY_WEIGHTS`` names the kernels that request weights there all the same, and why they may.
 
@@ -173,6 +175,12 @@ def lint_text(name: str, raw: str, multi_gpu: bool = True, helpers: Dict[str, st
         if POLL.search(header) or POLL.search(body):
             if not (BOUND.search(header) or BOUND.search(body)):
                 out.append({"rule": "bounded-wait", "file": name, "line": line, "what": "a polling loop without a time or iteration budget"})
+    for line, header, body in loops(text):
+        ld, own, inner = re.search(r"\btmem_ld\w*\s*\(", body), body, [b for _, _, b in loops(body)]
+        for b in inner:
+            own = own.replace(b, "")
+        if ld and re.search(r"\bcontinue\s*;", own) and not any("tmem_ld" in b for b in inner) and "__syncwarp(" not in body[: ld.start()]:
+            out.append({"rule": "converged", "file": name, "line": line, "what": "tensor memory loaded after a round that lanes may have left early, without __syncwarp"})
     for kname, body in kernels(text):
         if re.search(r"\btmem_alloc\s*\(", body) and not re.search(r"\btmem_dealloc\s*\(", body):
             out.append({"rule": "tmem-paired", "file": name, "line": 0, "what": f"kernel {kname} allocates tensor memory and never frees it"})

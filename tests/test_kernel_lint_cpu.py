@@ -48,3 +48,12 @@ def test_reads_in_front_of_the_dependency_wait():
     assert _rules(head + "{ out[0] = w[0]; }") == []                   # without a wait: launched in plain stream order
     named = [n for n, _, _ in kl.kernel_parts(kl.strip_comments(head + "{ }"))]
     assert named == ["k"]
+
+
+def test_warp_wide_loads_of_tensor_memory():
+    head = "__global__ void k(float* out) "
+    late = "tmem_ld_x16(t + c, r); tc_wait_ld(); if (!n_ok) continue; for (int j = 0; j < 16; ++j) out[j] = r[j]; } }"
+    assert _rules(head + "{ for (int c = 0; c < n; c += 16) { " + late) == ["converged"]
+    assert _rules(head + "{ for (int c = 0; c < n; c += 16) { __syncwarp(); " + late) == []
+    assert _rules(head + "{ for (int c = 0; c < n; c += 16) { tmem_ld_x16(t + c, r); for (int j = 0; j < 16; ++j) { if (j > m) continue; out[j] = r[j]; } } }") == []
+    assert _rules(head + "{ for (int i = 0; i < n; ++i) { if (!warp_wait(b)) continue; for (int c = 0; c < 4; ++c) { tmem_ld_x16(t + c, r); out[c] = r[0]; } } }") == []
