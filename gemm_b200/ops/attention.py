@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 import os
 from typing import Optional, Sequence
 
@@ -28,6 +29,11 @@ def _p(t):
 USE_DECODE_KERNEL = os.environ.get("GB_DECODE_ATTN", "1") != "0"      # 0: decode steps use the general kernel (A/B measurements)
 
 
+def whole_numbers(values) -> np.ndarray:
+    """Python integers, or integer scalars of numpy or torch on any device, as one int64 array; fractions are refused."""
+    return np.asarray([operator.index(v) for v in values], dtype=np.int64)
+
+
 def build_work(q_lens: Sequence[int], hq: int, hkv: int, num_splits: int = 1) -> torch.Tensor:
     """Host-side work list ``[n, 4] = {seq, kv_head, q_tok0, split}``: longest tiles first within a sequence,
     the heads of one tile adjacent (their K/V blocks hit in L2)."""
@@ -35,7 +41,7 @@ def build_work(q_lens: Sequence[int], hq: int, hkv: int, num_splits: int = 1) ->
     tpt = 128 // g
     if tpt == 0:                          # more query heads per KV head than a tile has rows: no work for the tcgen05 kernels
         return torch.zeros(0, 4, dtype=torch.int32)
-    tiles = np.maximum((np.asarray(q_lens, dtype=np.int64) + (tpt - 1)) // tpt, 0)
+    tiles = np.maximum((whole_numbers(q_lens) + (tpt - 1)) // tpt, 0)
     seq = np.repeat(np.arange(len(tiles)), tiles * (num_splits * hkv))
     at = np.arange(len(seq)) - np.repeat(np.cumsum(tiles) - tiles, tiles * (num_splits * hkv)) * (num_splits * hkv)       # item of its sequence: (tile, split, head)
     tile = tiles[seq] - 1 - at // (num_splits * hkv)

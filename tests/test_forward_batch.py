@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from gemm_b200.models.transformer import ForwardBatch
+from gemm_b200.ops import attention
 
 
 def _plain(q_lens, ctx, bt, page, all_logits):
@@ -53,3 +54,15 @@ def test_staged_layout():
         ForwardBatch.build([2, 1], [0, 5], [0, 1, 2], bt, 16, 8, 2, "cpu", stage=True)
     fb = ForwardBatch.build([1, 1, 1], [3, 4, 5], [0, 1, 2], bt, 16, 8, 2, "cpu", stage=True)
     assert fb.stage_slots.tolist() == [0, 1, 2] and fb.stage_bt is None
+
+
+def test_build_takes_whole_numbers_only():
+    bt = torch.zeros(2, 4, dtype=torch.int32)
+    for q_lens, ctx in (([2.5, 1], [0, 0]), ([2, 1], [0.5, 0]), ([2.0, 1.0], [0, 0])):
+        with pytest.raises(TypeError):
+            ForwardBatch.build(q_lens, ctx, [1, 2, 3], bt, 16, 8, 2, "cpu")
+    with pytest.raises(TypeError):
+        attention.build_work([2.5], 8, 2)
+    want = ForwardBatch.build([2, 1], [3, 0], [1, 2, 3], bt, 16, 8, 2, "cpu")
+    got = ForwardBatch.build(torch.tensor([2, 1]), torch.tensor([3, 0]), [1, 2, 3], bt, 16, 8, 2, "cpu")
+    assert got.positions.tolist() == want.positions.tolist() and got.work.tolist() == want.work.tolist()
