@@ -228,7 +228,7 @@ class ForwardBatch:
         parts = dict(positions=pos, slots=slots, cu_q=cu, kv_len=ctx + ql, work=att.build_work(q_lens, hq, hkv, num_splits).numpy(),
                      seq_slots=np.asarray([int(x) for x in seq_slots] if seq_slots is not None else range(b), dtype=np.int64))
         if block_table.device.type == "cpu" and torch.device(device).type != "cpu":
-            parts["block_table"] = block_table.numpy()
+            parts["block_table"] = block_table.to(torch.int32).numpy()         # (entries that no token uses may hold anything)
         if stage:
             if all(q == 1 for q in q_lens):
                 parts["stage_slots"] = np.arange(t)

@@ -66,3 +66,25 @@ def test_build_takes_whole_numbers_only():
     want = ForwardBatch.build([2, 1], [3, 0], [1, 2, 3], bt, 16, 8, 2, "cpu")
     got = ForwardBatch.build(torch.tensor([2, 1]), torch.tensor([3, 0]), [1, 2, 3], bt, 16, 8, 2, "cpu")
     assert got.positions.tolist() == want.positions.tolist() and got.work.tolist() == want.work.tolist()
+
+
+def _wide_table():
+    bt = torch.arange(12, dtype=torch.int64).view(2, 6)
+    bt[:, 4:] = 2 ** 40 + 7                               # entries past the sequences' pages: whatever the memory held
+    return bt
+
+
+def test_build_takes_tables_with_anything_in_unused_entries():
+    fb = ForwardBatch.build([20, 1], [10, 63], list(range(21)), _wide_table(), 16, 8, 2, "meta")
+    assert fb.block_table.shape == (2, 6) and fb.block_table.dtype == torch.int32
+
+
+@pytest.mark.gpu
+def test_build_on_the_device():
+    """One copy of all arrays to the GPU: the values of the CPU's batch, a table of 64-bit entries among them."""
+    args = ([20, 1], [10, 63], list(range(21)), _wide_table(), 16, 8, 2)
+    cpu, gpu = ForwardBatch.build(*args, "cpu", num_splits=2), ForwardBatch.build(*args, "cuda", num_splits=2)
+    for name in ("ids", "positions", "slots", "cu_q", "kv_len", "work", "seq_slots", "block_table", "logit_rows"):
+        a, b = getattr(cpu, name), getattr(gpu, name)
+        assert b.is_cuda and b.dtype == a.dtype and torch.equal(b.cpu(), a), name
+        assert b.data_ptr() % 16 == 0, name
