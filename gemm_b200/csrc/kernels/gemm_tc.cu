@@ -68,6 +68,7 @@ struct GemmArgs {
   // fp32 partial in sk_ws; the warp that arrives last at the tile's semaphore sums the partials in split order
   // (deterministic) and runs the normal epilogue.
   int splits;
+  int tok_group;                   // > 0: order of the plain launch's tiles (token_group)
   int tile_hint, m_tok_hint;       // host only: expected number of tiles and tokens per tile row (grid sizing of memory-bound launches)
   long partial_stride;             // > 0: no in-kernel reduction, split ks stores its fp32 partial at out + ks * partial_stride (elements)
   float* sk_ws;                    // [tiles][splits][NA * TN][128] fp32
@@ -91,6 +92,15 @@ struct GemmArgs {
 // k-steps whose MXFP8 scale atoms are fetched by one bulk copy (2 for the widest tile, whose stages are short of room)
 __host__ __device__ constexpr int sf_group(int tn) { return tn >= 256 ? 2 : tn >= 128 ? 4 : 1; }
 
+// Order of a plain launch's tiles: 0 = all blocks of features for a token tile before the next one, 8 = eight token tiles for a block before the next block.
+// With at least as many blocks as CTAs the first order streams the weights from memory once per token tile; in the second the eight tiles' rows stay in L2 (both
+// orders timed in turn, weights cold: 18944 features of 3584, 512 tokens 63.9 -> 59.2 us, 2048 tokens 248 -> 217 us; MXFP8, 51200 of 5120, 2048 tokens 589 -> 525 us;
+// 24576 pairs of 4096 with GELU, 2048 tokens 985 -> 788 us).  With fewer blocks a round covers several token tiles as it is.  The quantising epilogue is most of its
+// tile's time: with a ragged last tile every second or fourth CTA would get only such ones (25600 pairs of 5120, 400 tokens 369 -> 398 us, 512 tokens 407 -> 387 us).
+inline int token_group(int n_out, int m_tok, int tn, int splits, bool quant_out, int ctas) {
+  return splits <= 1 && m_tok > tn && (n_out + 127) / 128 >= ctas && (!quant_out || m_tok % tn == 0) ? 8 : 0;
+}
+
 struct Tile { int w_row0; int w_row1; int x_row0; int valid; int n0; int out_row0; int ks; int tile_id; };
 
 // Maps the linear tile index of the persistent loop to a tile.  Every warp role walks the same
@@ -107,11 +117,9 @@ struct TileCursor {
       if (t >= n_blocks * tok_blocks * sp) return false;
       o.ks = t % sp; o.tile_id = t / sp;
       int nb = o.tile_id % n_blocks, tb = o.tile_id / n_blocks;
-      if (sp == 1 && tok_blocks > 1 && n_blocks >= (int)gridDim.x) {
-        // at least as many blocks of features as CTAs: with all of them per token tile the weights would stream from memory once per tile.  Eight token tiles
-        // share a block instead, and their rows stay in L2 (16384 features, k = 4096: 512 tokens 93 -> 77 us, 2048 tokens 280 -> 251 us).
-        const int per = 8 * n_blocks, g = t / per, r = t - g * per, gt = min(8, tok_blocks - 8 * g);
-        nb = r / gt; tb = 8 * g + r % gt;
+      if (a.tok_group > 0) {               // that many token tiles share a block of features (token_group)
+        const int per = a.tok_group * n_blocks, g = t / per, r = t - g * per, gt = min(a.tok_group, tok_blocks - a.tok_group * g);
+        nb = r / gt; tb = a.tok_group * g + r % gt;
       }
       o.n0 = nb * 128; o.w_row0 = o.n0; o.w_row1 = a.up_row_offset + o.n0;
       o.x_row0 = tb * TN; o.valid = min(TN, a.m_tok - o.x_row0); o.out_row0 = o.x_row0;
@@ -695,7 +703,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             }
           }
         };
-        // Up to 32 columns leave TMEM in one load (20 and 32 tokens by 4096 features of 4096, three splits: 10.2 -> 10.0 us); wider tiles take 16 a round.
+        // Up to 32 columns leave TMEM in one load (32 tokens by 4096 features of 4096 in K splits: 10.1 -> 10.0 us); wider tiles take 16 a round.
         constexpr int COLS = TN <= 32 ? TN : 16;
 #pragma unroll 1
         for (int c = 0; c < TN; c += COLS) {
@@ -781,6 +789,7 @@ static int launch_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, GemmArgs 
       if (slots < best && slots * 100 < base * 97) { best = slots; grid = g; }      // worth it from 3 % fewer slots on
     }
   }
+  a.tok_group = a.num_groups == 0 ? token_group(a.n_out, a.m_tok, TN, a.splits, QUANT_OUT, grid) : 0;
   launch_k(kern, grid, kGemmThreads, smem, stream, tmW, tmX, a);
   GB_CUDA_OK(cudaGetLastError());
   return 0;
@@ -992,3 +1001,5 @@ GB_API int gb_gemm(const void* w, const void* x, void* out, int n_out, int k, in
 
 // Whether a SiLU gate / up projection of these sizes takes the pair kernel on a GPU of `sms` SMs (n_out a multiple of 256).
 GB_API int gb_gemm_takes_pairs(int n_out, int k, int m_tok, int sms) { return pair_pays(n_out, k, m_tok, sms) ? 1 : 0; }
+// Token tiles that share a block of features in the order of a plain launch's tiles on `sms` SMs (0: none do).
+GB_API int gb_gemm_token_group(int n_out, int m_tok, int tn, int quant_out, int sms) { return token_group(n_out, m_tok, tn, 1, quant_out != 0, sms); }

@@ -80,3 +80,40 @@ def test_gate_up_pairs_have_token_tiles_of_at_most_128():
         gemm.linear_swiglu(x, w, tn=256)
     with pytest.raises(RuntimeError, match="unsupported variant"):
         gemm.linear_swiglu(x, w, tn=256, act="gelu_tanh")
+
+
+def _mx(n, k):
+    w = mxfp8.quantize((torch.randn(n, k, device="cuda") * k ** -0.5).bfloat16())
+    return mxfp8.MxTensor(mxfp8.tile_weight(w.data), w.sf, w.rows, w.k, w.sf_layout, True)
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 18944, 64), (1300, 19200, 128), (2304, 18944, 72)])
+@pytest.mark.parametrize("form", ["gelu_tanh", "capped", "gelu"])
+def test_wide_layers_with_activations(m, n, k, form):
+    """With as many blocks of features as SMs several token tiles share a block: the same bits as a launch per token tile."""
+    x, w = _inputs(m, n if form == "gelu" else 2 * n, k)
+    call = (lambda v: gemm.linear(v, w, gelu=True, tn=256)) if form == "gelu" else (lambda v: gemm.linear_swiglu(v, w, tn=128, act=form, cap=7.0))
+    got = call(x)
+    _native.assert_status_ok()
+    for t in range(0, m, 256 if form == "gelu" else 128):
+        assert torch.equal(got[t: t + 128], call(x[t: t + 128])), t
+
+
+@pytest.mark.parametrize("m,k", [(300, 128), (512, 256), (2049, 128)])
+def test_wide_mxfp8_layers(m, k):
+    """The same for MXFP8 operands, plain and with the quantising epilogue (which keeps the other order with a ragged last tile)."""
+    torch.manual_seed(m)
+    n = 18944
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), _mx(n, k)
+    got = gemm.linear_mx(mxfp8.quantize(x), w, tn=256)
+    w2 = _mx(2 * n, k)
+    q = gemm.linear_mx_swiglu_quant(mxfp8.quantize(x), w2)
+    qe = mxfp8.unpack_sf_atoms(q.sf, q.data.shape[0], n // 32)
+    _native.assert_status_ok()
+    for t in range(0, m, 128):
+        xs = mxfp8.quantize(x[t: t + 128])
+        assert torch.equal(got[t: t + 128], gemm.linear_mx(xs, w, tn=256)), t
+        part = gemm.linear_mx_swiglu_quant(xs, w2)
+        rows = min(128, m - t)
+        assert torch.equal(q.data[t: t + rows], part.data[:rows]), t
+        assert torch.equal(qe[t: t + rows], mxfp8.unpack_sf_atoms(part.sf, part.data.shape[0], n // 32)[:rows]), t
