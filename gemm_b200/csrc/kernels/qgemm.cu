@@ -291,7 +291,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const QGemmArgs args) {
 // from there; what shared memory keeps free holds token tiles of up to 256, so W is unpacked once per 256 tokens.  Same operands, same order of sums as above.
 // 512 tokens by 51200 rows of 5120: 379 -> 247 us, by 5120 rows of 25600: 334 -> 188 us.
 //
-// TMEM: columns 0-255 accumulators (one of up to 256 columns, or two of up to 128), 256-511 four operand stages of 128 rows x 128 bf16 (64 columns each).
+// TMEM: columns 0-255 the accumulator (token tiles are wider than 128: two would not fit), 256-511 four operand stages of 128 rows x 128 bf16 (64 columns each).
 // Roles (864 threads): warp 0 producer of token tiles, warp 26 of raw tiles, warp 1 MMA issuer, warps 2-9 epilogue (token half (warp - 2) / 4), warps 10-25
 // unpack: two groups of eight take the raw tiles in turn (one group alone: 5 to 10 % more), and each fills its own two operand stages.
 constexpr int kQwThreads = 864;
@@ -302,7 +302,7 @@ __host__ __device__ constexpr int qw_raw_stages(int type) { return type == 0 ? 4
 
 struct QWideArgs {
   QGemmArgs g;
-  int tn;                                  // tokens of a tile: a multiple of 16, at most 256
+  int tn;                                  // tokens of a tile: a multiple of 16, from 144 to 256
 };
 
 template <int TYPE>
@@ -324,14 +324,13 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
   uint64_t* a_empty = a_full + kQwA;    // [kQwA]  1 (commit)
   uint64_t* b_full = a_empty + kQwA;    // [BS]
   uint64_t* b_empty = b_full + BS;      // [BS]  1 (commit)
-  uint64_t* accf = b_empty + BS;        // [2]
-  uint64_t* acce = accf + 2;            // [2]  8 arrivals (epilogue warps)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acce + 2);
+  uint64_t* accf = b_empty + BS;        // commit
+  uint64_t* acce = accf + 1;            // 8 arrivals (epilogue warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acce + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = args.row_tiles * args.tok_tiles * args.splits;
-  const int nacc = TN <= 128 ? 2 : 1;
   // token tiles vary fastest: the CTAs that run together share a tile of W
   auto tile_at = [&](int t, int& rt, int& tb, int& kb0, int& kb1) {
     const int ksp = t % args.splits, tt = t / args.splits;
@@ -344,7 +343,7 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
     for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
     for (int i = 0; i < kQwA; ++i) { mbar_init(&a_full[i], 8); mbar_init(&a_empty[i], 1); }
     for (int i = 0; i < BS; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&accf[i], 1); mbar_init(&acce[i], 8); }
+    mbar_init(accf, 1); mbar_init(acce, 8);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmX);
@@ -393,15 +392,14 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      int as = 0; uint32_t aph = 0; int bs = 0; uint32_t bph = 0; int acc = 0; uint32_t acc_ph = 0;
+      int as = 0; uint32_t aph = 0; int bs = 0; uint32_t bph = 0; uint32_t acc_ph = 0;
       bool ok = true;
       const uint32_t idesc = make_idesc(128, TN, 1, 1);
       for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
         int rt, tb, kb0, kb1;
         tile_at(t, rt, tb, kb0, kb1);
-        if (!mbar_wait(&acce[acc], acc_ph ^ 1, abort_flag, args.status, 1250, acc)) { ok = false; break; }
+        if (!mbar_wait(acce, acc_ph ^ 1, abort_flag, args.status, 1250)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + acc * 128;
         for (int ks = 0; ok && ks < 2 * (kb1 - kb0); ++ks) {
           if (!mbar_wait(&a_full[as], aph, abort_flag, args.status, 1251, as)) { ok = false; break; }
           for (int half = 0; half < 2; ++half) {
@@ -410,7 +408,7 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
             const uint64_t b = make_sdesc_sw128(smem_u32(Bb + bs * 32768));
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              mma_f16_ts(d0, tmem_a + as * 64 + half * 32 + j * 8, sdesc_at(b, j * 32), idesc, (ks > 0 || half > 0 || j > 0) ? 1u : 0u);
+              mma_f16_ts(tmem_base, tmem_a + as * 64 + half * 32 + j * 8, sdesc_at(b, j * 32), idesc, (ks > 0 || half > 0 || j > 0) ? 1u : 0u);
             tc_commit(&b_empty[bs]);
             if (++bs == BS) { bs = 0; bph ^= 1; }
           }
@@ -419,20 +417,20 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
           if (++as == kQwA) { as = 0; aph ^= 1; }
         }
         if (!ok) break;
-        tc_commit(&accf[acc]);
-        if (++acc == nacc) { acc = 0; acc_ph ^= 1; }
+        tc_commit(accf);
+        acc_ph ^= 1;
       }
     }
   } else if (warp < 10) {
     // ------------------------------------------------------------------ epilogue (warps 2..9)
     const int q = warp & 3, c0 = ((warp - 2) >> 2) * 128;
-    int acc = 0; uint32_t acc_ph = 0;
+    uint32_t acc_ph = 0;
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
       int rt, tb, kb0, kb1;
       const int ksp = tile_at(t, rt, tb, kb0, kb1);
-      if (!__all_sync(0xffffffffu, mbar_wait(&accf[acc], acc_ph, abort_flag, args.status, 1260, acc))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(accf, acc_ph, abort_flag, args.status, 1260))) break;
       tc_fence_after();
-      const uint32_t tacc = tmem_base + acc * 128 + c0 + ((uint32_t)(q * 32) << 16);
+      const uint32_t tacc = tmem_base + c0 + ((uint32_t)(q * 32) << 16);
       const int n = rt * 128 + q * 32 + lane;
       const bool n_ok = n < args.n_out;
       const float bias = (args.bias != nullptr && n_ok && ksp == 0) ? args.bias[n] : 0.f;
@@ -456,8 +454,8 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acce[acc]);
-      if (++acc == nacc) { acc = 0; acc_ph ^= 1; }
+      if (lane == 0) mbar_arrive(acce);
+      acc_ph ^= 1;
     }
   } else {
     // ------------------------------------------------------------------ unpack (warps 10..25): raw blocks -> operand in TMEM
@@ -553,8 +551,9 @@ qgemm_wide_kernel(const __grid_constant__ CUtensorMap tmX, const QWideArgs wargs
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-// Tokens of a tile of the wide kernel: the even cut of the tokens whose rounds of CTAs cost least.  A step of 128 k-columns costs much the same for any tile, a
-// little more for a wide one (512 tokens over 40 row tiles: three tiles of 176 tokens in one round).
+// Tokens of a tile of the wide kernel: the even cut of the tokens whose rounds of CTAs cost least, a step of 128 k-columns being a fixed part (the unpacking) and one per
+// token (51200 rows of 5120: 160 tokens 122 us in three rounds, 512 tokens 247 us in six; 512 tokens over 40 row tiles: three tiles of 176 tokens in one round).
+// At most 128: the narrow kernel's tiles do, see gb_qgemm.
 static int qgemm_wide_tn(int m, int row_tiles, int splits, int sms) {
   int best = 256;
   long best_cost = -1;
@@ -621,9 +620,9 @@ GB_API int gb_qgemm(const void* w, int ggml_type, const void* x, int ldx, void* 
   if (m <= 0) return 0;
   if (ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return fail("qgemm: operands must be 16-byte aligned%s");
   if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return fail("qgemm: token tile must be 16, 32, 64 or 128%s");
-  // A step of 128 k-columns takes the wide kernel about a tenth longer than the narrow one, whatever the tile's tokens: it is taken where its wider tiles save
-  // a round of CTAs (51200 rows of 5120: 128 tokens 107 us narrow, 117 wide; 160 tokens 204 and 122; 512 tokens 371 and 247; 5120 rows of 8192: 384 tokens 61
-  // and 65, 512 tokens 114 and 65).
+  // A step of 128 k-columns takes the wide kernel longer than the narrow one its 128 tokens (160 tokens 1.14 times, 256 tokens 1.22 times): it is taken where its
+  // tiles, which are fewer, save a round of CTAs; by these figures that pays at every size (51200 rows of 5120: 128 tokens 107 us narrow, 117 wide; 160 tokens 204
+  // and 122; 512 tokens 371 and 247; 5120 rows of 8192: 384 tokens 61 and 65, 512 tokens 114 and 65).  Tiles of at most 128 tokens cannot save one.
   bool wide = false;
   if (tn == 128) {
     const int row_tiles = (n_out + 127) / 128, sp = splits > 1 ? splits : 1, sms = sm_count(), wtn = qgemm_wide_tn(m, row_tiles, sp, sms);

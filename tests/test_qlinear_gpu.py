@@ -51,7 +51,7 @@ def test_gemm_matches_fp32_reference(t, rows, k, m):
 @pytest.mark.parametrize("rows,k,m", [(128, 256, 65), (200, 512, 80), (5120, 512, 129), (384, 2048, 256), (640, 768, 257), (5120, 1024, 512), (19072, 256, 300), (256, 5120, 1025),
                                       (10240, 512, 200), (10240, 768, 256), (24576, 1280, 450), (9500, 512, 161)])
 def test_gemm_wide_tiles(t, rows, k, m):
-    """More than 64 tokens, on both sides of the rule (tiles of 128, or the operand through TMEM and tiles of 16 to 256 where that saves a round of CTAs: 512 tokens
+    """More than 64 tokens, on both sides of the rule (tiles of 128, or the operand through TMEM and tiles of 144 to 256 where that saves a round of CTAs: 512 tokens
     of 5120 rows, 300 of 19072 and the last four).  Edges of tiles, one to many tiles per CTA, rings that wrap."""
     qw, x, ref = _case(t, rows, k, m, seed=rows + m)
     bias = torch.randn(rows, device="cuda")
