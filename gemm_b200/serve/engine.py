@@ -179,9 +179,10 @@ class Engine:
                 q_lens.append(take); ctx.append(done[i]); seqs.append(i)
                 ids.append(prompts[i][done[i]:done[i] + take])
                 room -= take
-            fb = ForwardBatch.build(q_lens, ctx, torch.cat(ids if all(x.device.type == "cpu" for x in ids) else [x.to(self.device) for x in ids]), self._block_table([base + i for i in seqs]),
-                                    self.page_size, self.hq_local, self.hkv_local, self.device, seq_slots=[base + i for i in seqs],
-                                    stage=self.kv.quantized)
+            on_host = all(x.device.type == "cpu" for x in ids)                 # then one copy to the device, of all of them
+            ids = torch.cat(ids if on_host else [x.to(self.device) for x in ids])
+            fb = ForwardBatch.build(q_lens, ctx, ids, self._block_table([base + i for i in seqs]), self.page_size, self.hq_local, self.hkv_local, self.device,
+                                    seq_slots=[base + i for i in seqs], stage=self.kv.quantized)
             if embeds is not None:
                 fb.embeds = torch.cat([embeds[i][c: c + q].to(self.device, torch.bfloat16) for i, c, q in zip(seqs, ctx, q_lens)])
                 if deepstack is not None and any(d is not None for d in deepstack):
