@@ -1,10 +1,12 @@
 """Token-wise, MoE-routing and sampling kernels vs their PyTorch fp32 references."""
+import ctypes
+
 import pytest
 import torch
 
 from gemm_b200 import _native
 from gemm_b200.ops import elementwise as ew
-from gemm_b200.ops import moe, mxfp8, quant, sampling
+from gemm_b200.ops import gemm, moe, mxfp8, quant, sampling
 
 pytestmark = pytest.mark.gpu
 
@@ -121,6 +123,103 @@ def test_qk_norm_rope_from_split_k_partials():
     q = ew.qk_norm_rope(pend, pos, slots, qw, kw, kc, vc, hq, hkv, d, 1e6, 1e-6, 0.25, None, table=tab)
     q2 = ew.qk_norm_rope(qkv, pos, slots, qw, kw, kc2, vc2, hq, hkv, d, 1e6, 1e-6, 0.25, None, table=tab)
     assert _rel(q, q2) < 6e-3 and _rel(kc, kc2) < 6e-3 and _rel(vc, vc2) < 6e-3
+
+
+def _slab_sum(parts):
+    """f32, slab by slab: the order in which the kernels add K-split partial sums."""
+    acc = torch.zeros_like(parts[0], dtype=torch.float32)
+    for p in parts:
+        acc = acc + p.float()
+    return acc
+
+
+# vectors of 8 per thread 1 to 4, whole and with threads of the last round idle; slabs below, at and past the groups that are loaded together
+@pytest.mark.parametrize("hidden", [256, 2048, 3080, 4096, 5120, 8192])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 8, 9])
+def test_rmsnorm_adds_slabs_in_order(hidden, n):
+    """The residual takes the slabs' f32 sum with one rounding, and the norm is that of the plain kernel: bit for bit."""
+    torch.manual_seed(hidden + n)
+    rows = 5
+    parts = torch.randn(n, rows, hidden, device="cuda") * 0.6
+    res = torch.randn(rows, hidden, device="cuda").bfloat16()
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda")).bfloat16()
+    want_res = (res.float() + _slab_sum(parts)).bfloat16()
+    want = ew.rmsnorm(want_res, w, 1e-6)
+    got_res = res.clone()
+    got = ew.rmsnorm(gemm.PendingPartials(parts), w, 1e-6, residual=got_res)
+    assert torch.equal(got_res, want_res) and torch.equal(got, want)
+    # the same sums as rows of bf16 (a reduce-scatter that travelled as such)
+    b16 = parts.bfloat16()
+    ctr = torch.zeros(2, dtype=torch.int32, device="cuda")
+    bc = ew.RmsBcast(partials_bf16=1, epoch_ctr=ctr.data_ptr(), done_ctr=ctr.data_ptr() + 4)          # (nowhere to gather to)
+    got_res, got = res.clone(), torch.empty_like(res)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    none, i = ctypes.c_void_p(0), ctypes.c_int
+    rc = _native.cuda().gb_rmsnorm_reduce_bcast(p(got_res), p(b16), i(n), ctypes.c_long(rows * hidden), p(w), p(got), none, none, i(rows), i(hidden), ctypes.c_float(1e-6), i(0),
+                                                none, i(0), none, ctypes.c_void_p(_native.status_ptr()), ctypes.byref(bc), ctypes.c_void_p(_native.stream()))
+    _native.check(rc, "gb_rmsnorm_reduce_bcast")
+    want_res = (res.float() + _slab_sum(b16)).bfloat16()
+    assert torch.equal(got_res, want_res) and torch.equal(got, ew.rmsnorm(want_res, w, 1e-6))
+
+
+@pytest.mark.parametrize("hidden", [2048, 5120])
+@pytest.mark.parametrize("ranks,splits", [(1, 3), (2, 1), (2, 3), (4, 2), (8, 3)])
+def test_rmsnorm_adds_ranks_and_splits_in_order(hidden, ranks, splits):
+    """Every rank's slot holds its K splits: ranks first, splits within them, the slots wider than their content."""
+    torch.manual_seed(ranks * 10 + splits)
+    rows = 6
+    slots = torch.randn(ranks, splits * rows * hidden + 64, device="cuda") * 0.5
+    parts = torch.cat([s[: splits * rows * hidden].view(splits, rows, hidden) for s in slots])
+    res = torch.randn(rows, hidden, device="cuda").bfloat16()
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda")).bfloat16()
+    want_res = (res.float() + _slab_sum(parts)).bfloat16()
+    got_res, got = res.clone(), torch.empty_like(res)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    none, i, l = ctypes.c_void_p(0), ctypes.c_int, ctypes.c_long
+    rc = _native.cuda().gb_rmsnorm_reduce2(p(got_res), p(slots), i(ranks), l(slots.shape[1]), i(splits), l(rows * hidden), p(w), p(got), none, none, i(rows), i(hidden),
+                                           ctypes.c_float(1e-6), i(0), none, i(0), none, ctypes.c_void_p(_native.status_ptr()), ctypes.c_void_p(_native.stream()))
+    _native.check(rc, "gb_rmsnorm_reduce2")
+    assert torch.equal(got_res, want_res) and torch.equal(got, ew.rmsnorm(want_res, w, 1e-6))
+
+
+@pytest.mark.parametrize("hidden", [256, 2048, 3080, 4096, 5120, 8192])
+@pytest.mark.parametrize("k", [1, 3, 6, 8])
+def test_rmsnorm_combines_experts_rows(hidden, k):
+    """The combine inside the norm against the combine kernel in front of it, bit for bit, some of the rows dropped."""
+    torch.manual_seed(hidden + k)
+    t, cap = 7, 64
+    y = torch.randn(cap, hidden, device="cuda").bfloat16()
+    rows = torch.randint(0, cap, (t, k), device="cuda", dtype=torch.int32)
+    rows[torch.rand(t, k, device="cuda") < 0.3] = -1
+    rows[0] = -1
+    wt = torch.rand(t, k, device="cuda")
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda")).bfloat16()
+    r1 = torch.randn(t, hidden, device="cuda").bfloat16()
+    r2 = r1.clone()
+    a = ew.rmsnorm(moe.combine(y, rows.view(-1), wt, t, k), w, 1e-6, residual=r1)
+    b = ew.rmsnorm(moe.PendingCombine(y, rows.view(-1), wt, t, k), w, 1e-6, residual=r2)
+    assert torch.equal(r1, r2) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 8, 9])
+def test_slabs_of_projections_are_added_in_order(n):
+    """Q / K norm and SiLU over K-split sums against the same kernel on the slabs' sum: bit for bit, groups of four slabs and remainders."""
+    torch.manual_seed(n)
+    t, hq, hkv, d = 9, 4, 2, 128
+    pos = torch.randint(0, 3000, (t,), device="cuda", dtype=torch.int32)
+    slots = torch.randperm(64, device="cuda")[:t].to(torch.int32)
+    qw, kw = ((1 + 0.1 * torch.randn(d, device="cuda")).bfloat16() for _ in range(2))
+    tab = ew.rope_table(3000, d, 1e6, "cuda")
+    parts = torch.randn(n, t, (hq + 2 * hkv) * d, device="cuda") * 0.6
+    out = []
+    for p in (parts, _slab_sum(parts)[None].contiguous()):
+        kc, vc = (torch.zeros(64, hkv, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        out.append((ew.qk_norm_rope(gemm.PendingPartials(p), pos, slots, qw, kw, kc, vc, hq, hkv, d, 1e6, 1e-6, 0.25, None, table=tab), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    for inter in (64, 1032):
+        parts = torch.randn(n, t, 2 * inter, device="cuda") * 2
+        a, b = (ew.silu_mul_partials(gemm.PendingPartials(p)) for p in (parts, _slab_sum(parts)[None].contiguous()))
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("lay_in,lay_out", [(128, 128), (128, 32), (32, 32)])
