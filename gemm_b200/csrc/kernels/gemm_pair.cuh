@@ -12,8 +12,8 @@
 // Roles of a CTA (320 threads): warp 0 producer (TMA; both CTAs' loads report to the leader's barrier), warp 1 MMA issuer (leader CTA only; its commits
 // arrive in both CTAs), warps 2-9 epilogue (lane quarter warp % 4, token half (warp - 2) / 4 of the CTA's own accumulators).  All waits are bounded.
 //
-// Tile order: eight token tiles (X of at most 2048 tokens, which stays in L2) are walked for one block of features before the next block, so that the weights
-// stream from memory once per 2048 tokens.
+// Tile order: eight token tiles (X of 8 tn tokens, at most 2048, which stay in L2) are walked for one block of features before the next block, so that the weights
+// stream from memory once per 8 tn tokens.
 #pragma once
 #include "sm100.cuh"
 #include "host_common.h"
